@@ -61,6 +61,33 @@ def test_gemm_wgrad_layout_and_accumulate(native, M, N, K):
     close(acc, 1.0 + 2.0 * ref, rtol=2e-2, atol=4e-2 * (M ** 0.5) * 0.25)
 
 
+# one shape or more per form of the kernel: pairs of CTAs with 256 and 128 columns, single CTAs with 128 and 64, divided
+# reductions; remainders in every dimension (N % 64 != 0 takes the unblocked MN-major copies)
+@pytest.mark.parametrize("M,N,K", [(2056, 5000, 136), (4104, 1096, 264), (776, 1032, 1032), (520, 264, 72), (264, 136, 2056), (72, 4088, 4104),
+                                   (8, 64, 512), (136, 8, 1544)])
+@pytest.mark.parametrize("layout", ["f", "d", "w"])
+def test_gemm_forms_at_tile_edges(native, M, N, K, layout):
+    a = rnd(*((K, M) if layout == "w" else (M, K)), seed=61)
+    b = rnd(*((N, K) if layout == "f" else (K, N)), seed=62)
+    A, B = a.double().t() if layout == "w" else a.double(), b.double().t() if layout == "f" else b.double()
+    ref = A @ B
+    slack = K * 2.0 ** -23 * (A.abs() @ B.abs())          # fp32 sums of K products in any order
+    run = lambda out, **kw: native.gemm(a, b, M, N, K, layout == "w", layout != "f", out, **kw)
+
+    def check(got, want, rounding):
+        bad = (got.double() - want).abs() > slack + rounding * want.abs() + 2.0 ** -23 * want.abs()
+        assert not bad.any(), f"{int(bad.sum())} of {bad.numel()} elements are out of bounds"
+
+    check(run(torch.full((M, N), float("nan"), dtype=torch.bfloat16, device="cuda")), ref, 2.0 ** -8)
+    check(run(torch.full((M, N), 3.0, dtype=torch.float32, device="cuda"), accumulate=True), ref + 3, 0.0)
+    bias = rnd(N, seed=63)
+    wide = torch.full((M, N + 3), 7.0, dtype=torch.float32, device="cuda")   # rows that TMA cannot store; neighbours untouched
+    check(run(wide[:, :N], bias=bias), ref + bias.double(), 0.0)
+    assert (wide[:, N:] == 7.0).all()
+    torch.cuda.synchronize()
+    assert native.read_status(clear=False) == 0
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("rows,H", [(37, 256), (128, 1600), (64, 4096), (16, 8192)])
 def test_norms(native, dtype, rows, H):
