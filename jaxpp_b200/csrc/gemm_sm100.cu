@@ -149,14 +149,18 @@ __device__ __forceinline__ void add_bias(float (&v)[32], const GemmParams& p, in
   }
 }
 
-// One row of 32 columns straight to memory: outputs whose rows are not 16-byte aligned.
+// One row of 32 columns straight to memory: outputs whose rows are not 16-byte aligned.  (Unrolled with a test per column:
+// a loop that ends at N would index `v` at run time and put it, and every step of the epilogue, into local memory: the
+// 128 x 256 outputs of a CTA then took 8000 cycles, longer than the products of 16 k blocks.)
 __device__ __forceinline__ void store_row(const float (&v)[32], const GemmParams& p, size_t row, int col0) {
   if (p.out_fp32) {
     float* d = static_cast<float*>(p.D) + row * p.ldd + col0;
-    for (int j = 0; j < 32 && col0 + j < p.N; ++j) d[j] = p.accumulate ? d[j] + v[j] : v[j];
+#pragma unroll
+    for (int j = 0; j < 32; ++j) if (col0 + j < p.N) d[j] = p.accumulate ? d[j] + v[j] : v[j];
   } else {
     __nv_bfloat16* d = static_cast<__nv_bfloat16*>(p.D) + row * p.ldd + col0;
-    for (int j = 0; j < 32 && col0 + j < p.N; ++j) d[j] = __float2bfloat16_rn(v[j]);
+#pragma unroll
+    for (int j = 0; j < 32; ++j) if (col0 + j < p.N) d[j] = __float2bfloat16_rn(v[j]);
   }
 }
 
@@ -396,10 +400,12 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
             *reinterpret_cast<uint4*>(part + r * BN + c * 32 + ((j ^ (r & 7)) << 2)) = make_uint4(w[4 * j], w[4 * j + 1], w[4 * j + 2], w[4 * j + 3]);
         }
       } else {
-        const bool any_row = row_w < p.M;
+        // A warp whose rows lie behind the last one stores nothing and must leave its buffers alone: without a store of its
+        // own to count, the wait for the store before last would not cover the last one, which may still be reading.
+        const int c_end = row_w < p.M ? BN : 0;
         const int cols = (p.out_fp32 || !p.tma_store) ? 32 : 64;      // columns per step: 128 bytes of a row
 #pragma unroll 1
-        for (int c = 0; c < BN; c += cols) {
+        for (int c = 0; c < c_end; c += cols) {
           const int col0 = n0 + c;
           if (col0 >= p.N) break;  // uniform across the warp
           uint32_t r[32];
@@ -439,7 +445,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
           }
           fence_proxy_async();
           __syncwarp();
-          if (lane == 0 && any_row) {
+          if (lane == 0) {
             if (p.accumulate) tma_reduce_add_3d(&map_d, b, col0, row_w, prob);
             else tma_store_3d(&map_d, b, col0, row_w, prob);
             bulk_commit();
@@ -622,11 +628,11 @@ static int num_sms() {
 
 // Which form a product takes.  A launch takes about  start + waves x (tile + k blocks x step);  the constants are
 // microseconds, fitted to runs of every form from 256^3 to 4096 x 32000 x 4096: a step of a pair costs half as much per
-// product as that of a single CTA (4096 x 12288 x 4096: 289 us with 256 x 256 pairs, 384 with 256 x 128 pairs; 4096^3:
-// 113, 147 and, for single CTAs, 171 with 128 x 128 and 285 with 128 x 64; the 128 x 256 tiles of one CTA used before
-// 155), but a large tile starts and ends slowly and leaves SMs idle when there are few of them (256^3: 12 us against 8
-// with 128 x 64 tiles; 1024 x 1600 x 1600: 18 us against 14).  Reductions are divided only where that leaves no CTA
-// without an SM, and down to eight k blocks per part (77 x 4096 x 11008: 47 us whole, 31 us in two parts).
+// product as that of a single CTA (4096 x 12288 x 4096: 269 us with 256 x 256 pairs, 341 with 256 x 128 pairs; 4096^3:
+// 100, 132 and, for single CTAs, 152 with 128 x 128 and 285 with 128 x 64; the 128 x 256 tiles of one CTA used before
+// 155), but a large tile starts and ends slowly and leaves SMs idle when there are few of them (256^3: 8.9 us against 7.4
+// with 128 x 64 tiles; 1024 x 1600 x 1600: 15 us against 12.5).  Reductions are divided only where that leaves no CTA
+// without an SM, and down to eight k blocks per part (77 x 4096 x 11008: 45 us whole, 31 us in two parts).
 enum Form { PAIR256, PAIR128, ONE128, ONE64, FORMS };
 struct Choice {
   int form, split;
@@ -634,7 +640,7 @@ struct Choice {
 static Choice choose(const GemmParams& p) {
   const int sms = num_sms();
   constexpr int tm[FORMS] = {256, 256, 128, 128}, tn[FORMS] = {256, 128, 128, 64}, ctas[FORMS] = {2, 2, 1, 1};
-  constexpr double start[FORMS] = {4.5, 3.0, 2.0, 1.0}, tile[FORMS] = {2.0, 1.5, 0.5, 0.3}, step[FORMS] = {0.40, 0.26, 0.385, 0.31};
+  constexpr double start[FORMS] = {4.5, 3.5, 3.0, 2.5}, tile[FORMS] = {0.7, 0.7, 0.3, 0.2}, step[FORMS] = {0.37, 0.255, 0.35, 0.31};
   const int k_blocks = (p.K + BK - 1) / BK;
   Choice best{PAIR256, 1};
   double best_t = 1e30;
