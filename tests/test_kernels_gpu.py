@@ -361,6 +361,37 @@ ATTN_CASES = [
 ]
 
 
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("B,Sq,Sk,H,Hkv,causal", [
+    (1, 1, 513, 2, 2, True), (2, 10, 10, 4, 2, True), (1, 129, 129, 2, 1, True), (1, 257, 640, 2, 2, False),
+    (1, 300, 100, 2, 2, True),      # the first 200 queries see no key at all
+    (3, 100, 300, 6, 2, True), (1, 769, 769, 4, 1, True), (9, 128, 128, 3, 3, False)])
+def test_flash_attention_at_block_edges(native, B, Sq, Sk, H, Hkv, causal, D):
+    """Pairs of query tiles of which one is empty or short, single and odd numbers of blocks, fully hidden rows, against
+    64 bits.  P and dS are rounded to bf16 before the second products (2^-9 each) and the results once more, so each
+    result is within 3 * 2^-8 of its 2-norm; the log-sum-exp is all fp32."""
+    q, k, v, do = rnd(B, Sq, H, D, seed=71), rnd(B, Sk, Hkv, D, seed=72), rnd(B, Sk, Hkv, D, seed=73), rnd(B, Sq, H, D, seed=74)
+    scale, G = D ** -0.5, H // Hkv
+    o, lse = native.attention(q, k, v, causal, scale)
+    got = native.attention_bwd(do, q, k, v, o, lse, causal, scale)
+    Q, K, V, dO = q.double(), k.double().repeat_interleave(G, 2), v.double().repeat_interleave(G, 2), do.double()
+    s = torch.einsum("bqhd,bkhd->bhqk", Q, K) * scale
+    if causal:
+        s = s.masked_fill(torch.arange(Sk, device="cuda")[None, :] > torch.arange(Sq, device="cuda")[:, None] + (Sk - Sq), float("-inf"))
+    rlse = torch.logsumexp(s, -1)
+    p = torch.exp(s - rlse[..., None]).nan_to_num(0.0)
+    ro = torch.einsum("bhqk,bkhd->bqhd", p, V)
+    ds = p * (torch.einsum("bqhd,bkhd->bhqk", dO, V) - (dO * ro).sum(-1).transpose(1, 2)[..., None]) * scale
+    fold = lambda t: t.view(B, Sk, Hkv, G, D).sum(3)
+    want = (torch.einsum("bhqk,bkhd->bqhd", ds, K), fold(torch.einsum("bhqk,bqhd->bkhd", ds, Q)), fold(torch.einsum("bhqk,bqhd->bkhd", p, dO)))
+    assert torch.equal(torch.isfinite(lse), torch.isfinite(rlse))
+    close(lse[torch.isfinite(rlse)], rlse[torch.isfinite(rlse)].float(), rtol=1e-5, atol=1e-5)
+    for a, b in ((o, ro), *zip(got, want)):
+        assert (a.double() - b).norm() <= 3 * 2.0 ** -8 * b.norm()
+    torch.cuda.synchronize()
+    assert native.read_status(clear=False) == 0
+
+
 @pytest.mark.parametrize("B,Sq,Sk,H,Hkv,D,causal", ATTN_CASES)
 def test_flash_attention_forward_backward(native, B, Sq, Sk, H, Hkv, D, causal):
     from jaxpp_b200.ops import attention as att
