@@ -181,26 +181,57 @@ def _route_ref(logits: Tensor, top_k: int):
 def _router_impl(logits: Tensor, top_k: int):
     from ..ops import core as _core
 
-    if _core._use_native(logits) and logits.dtype in (torch.float32, torch.bfloat16) and logits.shape[-1] <= 64 and top_k <= 8:
+    if _native_routing(logits, top_k):
+        return _router_native(logits, top_k, False)[:4]
+    return _route_ref(logits, top_k)
+
+
+def _native_routing(logits: Tensor, top_k: int) -> bool:
+    return (ops._use_native(logits) and logits.dtype in (torch.float32, torch.bfloat16) and logits.shape[-1] <= 64 and top_k <= 8)
+
+
+_bound = False
+
+
+def _native():
+    """The native library with the bindings of this module's kernels, and the module that holds it."""
+    global _bound
+    from ..ops import native
+
+    lib = native.load()
+    if not _bound:
         import ctypes
 
-        from ..ops import native
+        p, i, f = ctypes.c_void_p, ctypes.c_int, ctypes.c_float
+        lib.jpb_router.argtypes = [i, p, p, p, p, p, p, p, f, i, i, i, p]
+        lib.jpb_router_bwd.argtypes = [i, p, p, p, p, p, p, p, i, i, i, f, p]
+        lib.jpb_moe_slots.argtypes = [p, p, p, p, i, i, i, p]
+        lib.jpb_moe_dispatch_rows.argtypes = [i, p, p, p, i, i, i, p]
+        lib.jpb_moe_combine_rows.argtypes = [i, p, p, p, p, i, i, i, i, p]
+        lib.jpb_moe_combine_rows_bwd.argtypes = [i, p, p, p, p, p, p, i, i, i, p]
+        _bound = True
+    return lib, native
 
-        lib = native.load()
-        p, i = ctypes.c_void_p, ctypes.c_int
-        lib.jpb_router.argtypes = [i, p, p, p, p, p, p, i, i, i, p]
-        lg = logits.contiguous()
-        T, E = lg.shape
-        dev = lg.device
-        probs = torch.empty(T, E, dtype=torch.float32, device=dev)
-        top_i = torch.empty(T, top_k, dtype=torch.int64, device=dev)
-        weights = torch.empty(T, top_k, dtype=torch.float32, device=dev)
-        stats = torch.empty(2, E, dtype=torch.float32, device=dev)
-        native._check(lib.jpb_router(0 if lg.dtype == torch.float32 else 1, lg.data_ptr(), probs.data_ptr(), top_i.data_ptr(),
-                                     weights.data_ptr(), stats[0].data_ptr(), stats[1].data_ptr(), T, E, top_k,
-                                     native._stream()), "jpb_router")
-        return top_i, weights, probs, stats[1]
-    return _route_ref(logits, top_k)
+
+def _aux_scale(T: int, E: int, top_k: int) -> float:
+    """aux = E * sum_e (hits_e / (T k)) * mean_t probs[t, e] = _aux_scale * sum_e hits_e * sum_t probs[t, e]"""
+    return E / (T * top_k * T) if T else float("nan")
+
+
+def _router_native(logits: Tensor, top_k: int, want_aux: bool):
+    lib, native = _native()
+    lg = logits.contiguous()
+    T, E = lg.shape
+    dev = lg.device
+    probs = torch.empty(T, E, dtype=torch.float32, device=dev)
+    top_i = torch.empty(T, top_k, dtype=torch.int64, device=dev)
+    weights = torch.empty(T, top_k, dtype=torch.float32, device=dev)
+    stats = torch.empty(2, E, dtype=torch.float32, device=dev)
+    aux = torch.empty((), dtype=torch.float32, device=dev) if want_aux else None
+    native._check(lib.jpb_router(native._dt(lg), lg.data_ptr(), probs.data_ptr(), top_i.data_ptr(), weights.data_ptr(),
+                                 stats.data_ptr(), stats.data_ptr() + 4 * E, native._p(aux), _aux_scale(T, E, top_k), T, E, top_k,
+                                 native._stream()), "jpb_router", 2 if want_aux else 1)
+    return top_i, weights, probs, stats[1], aux
 
 
 _lib.define("router(Tensor logits, int top_k) -> (Tensor, Tensor, Tensor, Tensor)")
@@ -225,6 +256,10 @@ def _router_setup(ctx, inputs, output):
 def _router_bwd(ctx, g_idx, g_w, g_probs, g_hits):
     """weights_j = p_{i_j} / S with S the sum of the picked probabilities; probs = softmax(logits)."""
     top_i, probs = ctx.saved_tensors
+    return _logits_grad(top_i, probs, g_w, g_probs).to(ctx.in_dtype), None
+
+
+def _logits_grad(top_i: Tensor, probs: Tensor, g_w, g_probs) -> Tensor:
     dp = g_probs.float() if g_probs is not None else torch.zeros_like(probs)
     if g_w is not None:
         pv = probs.gather(1, top_i)
@@ -232,21 +267,65 @@ def _router_bwd(ctx, g_idx, g_w, g_probs, g_hits):
         gw = g_w.float()
         d_pv = gw / s - (gw * pv).sum(-1, keepdim=True) / (s * s)
         dp = dp.scatter_add(1, top_i, d_pv)
-    dlogits = probs * (dp - (dp * probs).sum(-1, keepdim=True))
-    return dlogits.to(ctx.in_dtype), None
+    return probs * (dp - (dp * probs).sum(-1, keepdim=True))
 
 
 torch.library.register_autograd("b200moe::router", _router_bwd, setup_context=_router_setup)
 
 
+# The router together with the load-balancing loss: one op each way instead of the router and a dozen small reductions
+# and elementwise ops around it (launches, not work, are the cost of routing).
+def _route_tokens_impl(logits: Tensor, top_k: int):
+    if _native_routing(logits, top_k):
+        return _router_native(logits, top_k, True)
+    top_i, weights, probs, hits = _route_ref(logits, top_k)
+    frac = hits / (top_i.shape[0] * top_k)
+    return top_i, weights, probs, hits, logits.shape[-1] * (frac * probs.mean(0)).sum()
+
+
+def _route_tokens_bwd_impl(top_i: Tensor, probs: Tensor, hits: Tensor, g_w, g_probs, g_aux, like: Tensor) -> Tensor:
+    T, E = probs.shape
+    k = top_i.shape[1]
+    if _native_routing(like, k):
+        lib, native = _native()
+        gs = [None if g is None else g.float().contiguous() for g in (g_w, g_probs, g_aux)]
+        out = torch.empty(T, E, dtype=like.dtype, device=like.device)
+        native._check(lib.jpb_router_bwd(native._dt(like), top_i.contiguous().data_ptr(), probs.contiguous().data_ptr(), native._p(gs[0]),
+                                         native._p(gs[1]), native._p(gs[2]), hits.contiguous().data_ptr(), out.data_ptr(), T, E, k,
+                                         _aux_scale(T, E, k), native._stream()), "jpb_router_bwd")
+        return out
+    if g_aux is not None:
+        d_aux = (g_aux.float() * _aux_scale(T, E, k) * hits).expand_as(probs)
+        g_probs = d_aux if g_probs is None else g_probs.float() + d_aux
+    return _logits_grad(top_i, probs, g_w, g_probs).to(like.dtype)
+
+
+_lib.define("route_tokens(Tensor logits, int top_k) -> (Tensor, Tensor, Tensor, Tensor, Tensor)")
+_lib.impl("route_tokens", _route_tokens_impl, "CompositeExplicitAutograd")
+_lib.define("route_tokens_bwd(Tensor top_i, Tensor probs, Tensor hits, Tensor? g_w, Tensor? g_probs, Tensor? g_aux, Tensor like) -> Tensor")
+_lib.impl("route_tokens_bwd", _route_tokens_bwd_impl, "CompositeExplicitAutograd")
+torch.library.register_fake("b200moe::route_tokens", lambda logits, top_k: (
+    *_router_fake(logits, top_k), torch.empty((), dtype=torch.float32, device=logits.device)))
+torch.library.register_fake("b200moe::route_tokens_bwd", lambda top_i, probs, hits, g_w, g_probs, g_aux, like: torch.empty(
+    probs.shape, dtype=like.dtype, device=like.device))
+
+
+def _route_tokens_setup(ctx, inputs, output):
+    ctx.save_for_backward(output[0], output[2], output[3], inputs[0])
+
+
+def _route_tokens_bwd(ctx, g_idx, g_w, g_probs, g_hits, g_aux):
+    top_i, probs, hits, logits = ctx.saved_tensors
+    return torch.ops.b200moe.route_tokens_bwd(top_i, probs, hits, g_w, g_probs, g_aux, logits), None
+
+
+torch.library.register_autograd("b200moe::route_tokens", _route_tokens_bwd, setup_context=_route_tokens_setup)
+
+
 def route(x: Tensor, w_router: Tensor, top_k: int):
     """Returns (expert ids [T,k] int64, weights [T,k] fp32, aux loss scalar fp32).  Softmax, top-k, renormalised
-    weights and the load-balancing statistics come from one kernel on the GPU (``b200moe::router``)."""
-    logits = ops.linear(x, w_router, None)
-    top_i, weights, probs, hits = torch.ops.b200moe.router(logits, top_k)
-    E = w_router.shape[0]
-    frac = hits / (top_i.shape[0] * top_k)
-    aux = E * (frac.detach() * probs.mean(0)).sum()
+    weights and the load-balancing loss come from one op (``b200moe::route_tokens``)."""
+    top_i, weights, _, _, aux = torch.ops.b200moe.route_tokens(ops.linear(x, w_router, None), top_k)
     return top_i, weights, aux
 
 
@@ -288,6 +367,128 @@ def combine(y_buf: Tensor, dest: Tensor, weights: Tensor, top_k: int) -> Tensor:
     return (picked.float() * weights.unsqueeze(-1)).sum(1).to(y_buf.dtype)
 
 
+# ---- the same three steps as kernels, where the experts are on this device -------------------------------------------
+# ``inv`` [E * C] int32 names the pick that fills each slot (-1: none), so that both directions are gathers: a slot's row
+# is written once, zeros included, and no gradient is accumulated with atomics.
+def _slots_impl(top_i: Tensor, n_experts: int, capacity: int):
+    n = top_i.numel()
+    if ops._use_native(top_i) and top_i.dtype == torch.int64 and n_experts <= 64 and n_experts * capacity < 2 ** 31:
+        lib, native = _native()
+        flat = top_i.contiguous()
+        dest = torch.empty(n, dtype=torch.int64, device=flat.device)
+        inv = torch.empty(n_experts * capacity, dtype=torch.int32, device=flat.device)
+        counts = torch.empty(n_experts, dtype=torch.int32, device=flat.device)
+        native._check(lib.jpb_moe_slots(flat.data_ptr(), dest.data_ptr(), inv.data_ptr(), counts.data_ptr(), n, n_experts, capacity,
+                                        native._stream()), "jpb_moe_slots")
+        return dest, inv, counts
+    dest, _, counts = slots_and_counts(top_i, n_experts, capacity)
+    inv = torch.full((n_experts * capacity + 1,), -1, dtype=torch.int32, device=dest.device)
+    inv[dest] = torch.arange(n, device=dest.device, dtype=torch.int32)
+    return dest, inv[:-1].clone(), counts
+
+
+def _rows_native(t: Tensor, *others) -> bool:
+    return (ops._use_native(t) and t.dtype in (torch.float32, torch.bfloat16) and t.shape[-1] % (16 // t.element_size()) == 0
+            and all(o is None or o.dtype == torch.float32 for o in others))
+
+
+def _row_operand(t: Tensor) -> Tensor:
+    t = t.contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
+def _dispatch_rows_impl(x: Tensor, dest: Tensor, inv: Tensor, top_k: int) -> Tensor:
+    slots, d = inv.numel(), x.shape[-1]
+    if _rows_native(x):
+        lib, native = _native()
+        x = _row_operand(x)
+        out = torch.empty(slots, d, dtype=x.dtype, device=x.device)
+        native._check(lib.jpb_moe_dispatch_rows(native._dt(x), x.data_ptr(), inv.contiguous().data_ptr(), out.data_ptr(), slots, d, top_k,
+                                           native._stream()), "jpb_moe_dispatch_rows")
+        return out
+    rows = x.index_select(0, (inv.clamp(min=0) // top_k).long())
+    return torch.where((inv >= 0).unsqueeze(-1), rows, torch.zeros_like(rows))
+
+
+def _combine_rows_impl(y: Tensor, dest: Tensor, inv: Tensor, weights, top_k: int) -> Tensor:
+    slots, d = y.shape
+    T = dest.numel() // top_k
+    if _rows_native(y, weights):
+        lib, native = _native()
+        y = _row_operand(y)
+        w = None if weights is None else weights.contiguous()
+        out = torch.empty(T, d, dtype=y.dtype, device=y.device)
+        native._check(lib.jpb_moe_combine_rows(native._dt(y), y.data_ptr(), dest.contiguous().data_ptr(), native._p(w), out.data_ptr(), T, d,
+                                          top_k, slots, native._stream()), "jpb_moe_combine_rows")
+        return out
+    flat = torch.cat([y, torch.zeros(1, d, dtype=y.dtype, device=y.device)], 0)
+    picked = flat.index_select(0, dest).view(T, top_k, d).float()
+    return (picked if weights is None else picked * weights.view(T, top_k, 1)).sum(1).to(y.dtype)
+
+
+def _combine_rows_bwd_impl(g: Tensor, y: Tensor, dest: Tensor, inv: Tensor, weights: Tensor, top_k: int):
+    slots, d = y.shape
+    T = dest.numel() // top_k
+    if _rows_native(y, weights) and g.dtype == y.dtype:
+        lib, native = _native()
+        g, y, w = _row_operand(g), _row_operand(y), weights.contiguous()
+        dy = torch.empty_like(y)
+        dw = torch.zeros(T * top_k, dtype=torch.float32, device=y.device)
+        native._check(lib.jpb_moe_combine_rows_bwd(native._dt(y), g.data_ptr(), y.data_ptr(), inv.contiguous().data_ptr(), w.data_ptr(),
+                                              dy.data_ptr(), dw.data_ptr(), slots, d, top_k, native._stream()), "jpb_moe_combine_rows_bwd")
+        return dy, dw
+    flat = torch.cat([y, torch.zeros(1, d, dtype=y.dtype, device=y.device)], 0)
+    rows = g.float().repeat_interleave(top_k, 0)
+    dw = (flat.index_select(0, dest).float() * rows).sum(-1)
+    dy = torch.zeros_like(flat).index_copy(0, dest, (rows * weights.reshape(-1, 1)).to(y.dtype))[:-1].clone()
+    return dy, dw.to(weights.dtype)
+
+
+_lib.define("slots(Tensor top_i, int n_experts, int capacity) -> (Tensor, Tensor, Tensor)")
+_lib.impl("slots", _slots_impl, "CompositeExplicitAutograd")
+_lib.define("dispatch_rows(Tensor x, Tensor dest, Tensor inv, int top_k) -> Tensor")
+_lib.impl("dispatch_rows", _dispatch_rows_impl, "CompositeExplicitAutograd")
+_lib.define("combine_rows(Tensor y, Tensor dest, Tensor inv, Tensor? weights, int top_k) -> Tensor")
+_lib.impl("combine_rows", _combine_rows_impl, "CompositeExplicitAutograd")
+_lib.define("combine_rows_bwd(Tensor g, Tensor y, Tensor dest, Tensor inv, Tensor weights, int top_k) -> (Tensor, Tensor)")
+_lib.impl("combine_rows_bwd", _combine_rows_bwd_impl, "CompositeExplicitAutograd")
+torch.library.register_fake("b200moe::slots", lambda top_i, n_experts, capacity: (
+    torch.empty(top_i.numel(), dtype=torch.int64, device=top_i.device),
+    torch.empty(n_experts * capacity, dtype=torch.int32, device=top_i.device),
+    torch.empty(n_experts, dtype=torch.int32, device=top_i.device)))
+torch.library.register_fake("b200moe::dispatch_rows", lambda x, dest, inv, top_k: x.new_empty(inv.shape[0], x.shape[-1]))
+torch.library.register_fake("b200moe::combine_rows", lambda y, dest, inv, weights, top_k: y.new_empty(dest.shape[0] // top_k, y.shape[-1]))
+torch.library.register_fake("b200moe::combine_rows_bwd", lambda g, y, dest, inv, weights, top_k: (
+    torch.empty_like(y, memory_format=torch.contiguous_format), weights.new_empty(dest.shape[0])))
+
+
+def _dispatch_rows_setup(ctx, inputs, output):
+    _, dest, inv, ctx.top_k = inputs
+    ctx.save_for_backward(dest, inv)
+
+
+def _dispatch_rows_bwd(ctx, g):
+    dest, inv = ctx.saved_tensors
+    return torch.ops.b200moe.combine_rows(g.contiguous(), dest, inv, None, ctx.top_k), None, None, None
+
+
+def _combine_rows_setup(ctx, inputs, output):
+    y, dest, inv, weights, ctx.top_k = inputs
+    ctx.save_for_backward(y if weights is not None else None, dest, inv, weights)
+
+
+def _combine_rows_bwd(ctx, g):
+    y, dest, inv, weights = ctx.saved_tensors
+    if weights is None:
+        return torch.ops.b200moe.dispatch_rows(g.contiguous(), dest, inv, ctx.top_k), None, None, None, None
+    dy, dw = torch.ops.b200moe.combine_rows_bwd(g.contiguous(), y, dest, inv, weights, ctx.top_k)
+    return dy, None, None, dw, None
+
+
+torch.library.register_autograd("b200moe::dispatch_rows", _dispatch_rows_bwd, setup_context=_dispatch_rows_setup)
+torch.library.register_autograd("b200moe::combine_rows", _combine_rows_bwd, setup_context=_combine_rows_setup)
+
+
 def expert_ffn(x: Tensor, w_up: Tensor, w_down: Tensor, counts: Tensor | None = None, seg_rows: int = 0) -> Tensor:
     """x: [E_l, M, d]; w_up: [E_l, 2F, d] ([gate | up]); w_down: [E_l, d, F].  Every local expert has room for the
     same number of slots, so each projection is one grouped tcgen05 GEMM over all local experts.  ``counts``
@@ -306,20 +507,23 @@ def moe_ffn(x: Tensor, p: dict, n_experts: int, top_k: int, capacity_factor: flo
     from ..utils import config
 
     top_i, weights, aux = route(x, p["router"], top_k)
+    if ep == 1:
+        dest, inv, counts = torch.ops.b200moe.slots(top_i, n_experts, capacity)
+        counts = counts.view(n_experts, 1) if config.moe_skip_empty_slots.value > 0 else None
+        buf = torch.ops.b200moe.dispatch_rows(x, dest, inv, top_k).view(n_experts, capacity, d)
+        y = expert_ffn(buf, p["w_up"], p["w_down"], counts, capacity)
+        return torch.ops.b200moe.combine_rows(y.reshape(n_experts * capacity, d), dest, inv, weights.reshape(-1), top_k), aux
     dest, _, counts = slots_and_counts(top_i, n_experts, capacity)
     if config.moe_skip_empty_slots.value <= 0:
         counts = None
-    if ep > 1:
-        buf = torch.ops.b200moe.dispatch_a2a(x, dest, None, n_experts, capacity, top_k, ep_axis)   # [E_l, ep*C, d]
-        if counts is not None:
-            # every rank tells the owner of each expert how many of its C slots it filled: [ep (source), E_l] -> [E_l, ep]
-            counts = torch.ops.b200moe.all_to_all(counts.view(ep, n_experts // ep), ep_axis).t().contiguous()
-        y = expert_ffn(buf, p["w_up"], p["w_down"], counts, capacity)
-        out, _ = torch.ops.b200moe.combine_a2a(y, dest, weights.reshape(-1), n_experts, capacity, top_k, ep_axis, True)
-        return out, aux
-    buf = dispatch(x, dest, n_experts, capacity, top_k)                        # [E, C, d]
-    y = expert_ffn(buf, p["w_up"], p["w_down"], None if counts is None else counts.view(n_experts, 1), capacity)
-    return combine(y.reshape(n_experts, capacity, d), dest, weights, top_k), aux
+    buf = torch.ops.b200moe.dispatch_a2a(x, dest, None, n_experts, capacity, top_k, ep_axis)   # [E_l, ep*C, d]
+    if counts is not None:
+        # every rank tells the owner of each expert how many of its C slots it filled: [ep (source), E_l] -> [E_l, ep]
+        counts = torch.ops.b200moe.all_to_all(counts.view(ep, n_experts // ep), ep_axis).t().contiguous()
+    y = expert_ffn(buf, p["w_up"], p["w_down"], counts, capacity)
+    out, _ = torch.ops.b200moe.combine_a2a(y, dest, weights.reshape(-1), n_experts, capacity, top_k, ep_axis, True)
+    return out, aux
+
 
 def _register_direct_calls():
     """Generated task code calls these implementations without the dispatcher (see ops.core.DIRECT)."""
@@ -329,6 +533,12 @@ def _register_direct_calls():
     _core.DIRECT[torch.ops.b200moe.dispatch_a2a.default] = _dispatch_a2a_impl
     _core.DIRECT[torch.ops.b200moe.combine_a2a.default] = _combine_a2a_impl
     _core.DIRECT[torch.ops.b200moe.router.default] = _router_impl
+    _core.DIRECT[torch.ops.b200moe.route_tokens.default] = _route_tokens_impl
+    _core.DIRECT[torch.ops.b200moe.route_tokens_bwd.default] = _route_tokens_bwd_impl
+    _core.DIRECT[torch.ops.b200moe.slots.default] = _slots_impl
+    _core.DIRECT[torch.ops.b200moe.dispatch_rows.default] = _dispatch_rows_impl
+    _core.DIRECT[torch.ops.b200moe.combine_rows.default] = _combine_rows_impl
+    _core.DIRECT[torch.ops.b200moe.combine_rows_bwd.default] = _combine_rows_bwd_impl
 
 
 _register_direct_calls()

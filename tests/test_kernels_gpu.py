@@ -264,6 +264,59 @@ def test_router_kernel(native, dtype):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("T,E,k,C,d", [(1000, 8, 2, 256, 512), (77, 16, 4, 8, 40), (3000, 64, 1, 40, 264), (1, 4, 2, 8, 8), (1025, 4, 3, 800, 4096)])
+def test_moe_row_kernels_match_the_composition(native, T, E, k, C, d, dtype):
+    """Slots, dispatch, combination and their gradients as kernels against the index ops they stand for: slots, copies and
+    scaled copies are the same bits, sums over at most k (or d) fp32 products differ by their rounding."""
+    from jaxpp_b200.parallel import moe
+
+    g = torch.Generator().manual_seed(5)
+    top_i = torch.stack([torch.randperm(E, generator=g)[:k] for _ in range(T)]).cuda()
+    dest, _, counts = moe.slots_and_counts(top_i, E, C)
+    d2, inv, c2 = torch.ops.b200moe.slots(top_i, E, C)
+    assert torch.equal(dest, d2) and torch.equal(counts, c2)
+    x, y, go = rnd(T, d, dtype=dtype, seed=81), rnd(E * C, d, dtype=dtype, seed=82), rnd(T, d, dtype=dtype, seed=83)
+    w = torch.rand(T * k, generator=g).cuda()
+    buf = torch.ops.b200moe.dispatch_rows(x, dest, inv, k)
+    assert torch.equal(buf.view(E, C, d), moe.dispatch(x, dest, E, C, k))
+    half = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -22
+    yd = torch.cat([y, y.new_zeros(1, d)]).double()
+    want = (yd[dest].view(T, k, d) * w.double().view(T, k, 1)).sum(1)
+    slack = (yd[dest].abs().view(T, k, d) * w.double().view(T, k, 1)).sum(1) * k * 2.0 ** -23
+    assert ((torch.ops.b200moe.combine_rows(y, dest, inv, w, k).double() - want).abs() <= slack + half * want.abs()).all()
+    dy, dw = torch.ops.b200moe.combine_rows_bwd(go, y, dest, inv, w, k)
+    rows = (go.float().repeat_interleave(k, 0) * w[:, None]).to(dtype)
+    ref = torch.zeros(E * C + 1, d, dtype=dtype, device="cuda")
+    ref[dest] = rows
+    assert torch.equal(dy, ref[:-1])
+    prod = yd[dest] * go.double().repeat_interleave(k, 0)
+    assert ((dw.double() - prod.sum(-1)).abs() <= d * 2.0 ** -23 * prod.abs().sum(-1)).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("T,E,k", [(1000, 8, 2), (65, 5, 1), (130, 17, 8), (33, 64, 3)])
+def test_route_tokens_kernel_matches_the_composition(native, T, E, k, dtype):
+    from jaxpp_b200.parallel import moe
+
+    logits = rnd(T, E, dtype=dtype, seed=91)
+    gw = torch.rand(T, k, device="cuda")
+    ti, w, probs, hits, aux = torch.ops.b200moe.route_tokens(logits, k)
+    lg = logits.double().requires_grad_(True)
+    p = torch.softmax(lg, -1)
+    pv = p.gather(1, ti)
+    rw = pv / pv.sum(-1, keepdim=True)
+    raux = E * (hits.double() / (T * k) * p.mean(0)).sum()
+    assert torch.equal(ti.sort(-1).values, torch.topk(logits.float(), k).indices.sort(-1).values)
+    assert torch.equal(hits, torch.bincount(ti.reshape(-1), minlength=E).float())
+    close(w, rw.float(), rtol=1e-5, atol=1e-6)
+    close(aux, raux.float(), rtol=1e-5, atol=1e-6)
+    (want,) = torch.autograd.grad((rw * gw).sum() + 3.0 * raux, [lg])
+    got = torch.ops.b200moe.route_tokens_bwd(ti, probs, hits, gw, None, torch.tensor(3.0, device="cuda"), logits)
+    bound = 2.0 ** -8 if dtype == torch.bfloat16 else 1e-5
+    assert (got.double() - want).norm() <= bound * want.norm()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_dropout_matches_counter_based_reference(native, dtype):
     from jaxpp_b200.ops import core as ops
 

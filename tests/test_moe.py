@@ -1,4 +1,5 @@
 """Mixture-of-experts building blocks on CPU: routing, capacity slots, dispatch / combine and their transposes."""
+import pytest
 import torch
 
 import jaxpp_b200 as jp
@@ -134,3 +135,39 @@ def test_router_op_backward_matches_autograd_of_the_composition():
     (gb,) = torch.autograd.grad(lb, [b])
     assert torch.equal(ia, ib) and torch.equal(ha, hb) and hb.sum().item() == T * k
     torch.testing.assert_close(gb, ga, rtol=1e-5, atol=1e-6)
+
+
+@pytest.mark.parametrize("T,d,E,k,C", [(33, 16, 4, 2, 12), (20, 8, 8, 1, 8), (7, 8, 4, 3, 64)])
+def test_row_ops_and_route_tokens_match_the_composition(T, d, E, k, C):
+    """The ops of the single-device path against dispatch / combine / router and the loss formula, with gradients."""
+    g = torch.Generator().manual_seed(0)
+    top = torch.stack([torch.randperm(E, generator=g)[:k] for _ in range(T)])
+    x, w, gw = torch.randn(T, d, generator=g), torch.rand(T * k, generator=g), torch.rand(T, k, generator=g)
+    dest, _, counts = moe.slots_and_counts(top, E, C)
+    d2, inv, c2 = torch.ops.b200moe.slots(top, E, C)
+    assert torch.equal(dest, d2) and torch.equal(counts, c2)
+
+    def composed(x, w):
+        b = moe.dispatch(x, dest, E, C, k)
+        return moe.combine(torch.sin(b) + b * b, dest, w.view(T, k), k)
+
+    def rows(x, w):
+        b = torch.ops.b200moe.dispatch_rows(x, dest, inv, k)
+        return torch.ops.b200moe.combine_rows(torch.sin(b) + b * b, dest, inv, w, k)
+
+    def composed_router(lg):
+        ti, wt, pr, h = torch.ops.b200moe.router(lg, k)
+        return (wt * gw).sum() + 2 * E * ((h / (T * k)).detach() * pr.mean(0)).sum()
+
+    def one_op(lg):
+        ti, wt, pr, h, aux = torch.ops.b200moe.route_tokens(lg, k)
+        return (wt * gw).sum() + 2 * aux
+
+    for fns, args in (((composed, rows), (x, w)), ((composed_router, one_op), (torch.randn(T, E, generator=g),))):
+        results = []
+        for f in fns:
+            leaves = [a.clone().requires_grad_(True) for a in args]
+            out = f(*leaves)
+            results.append((out, *torch.autograd.grad((out * torch.cos(out.detach())).sum(), leaves)))
+        for a, b in zip(*results):
+            torch.testing.assert_close(a, b)
