@@ -267,35 +267,43 @@ __global__ void __launch_bounds__(MAXT) norm_bwd_kernel(const T* __restrict__ dy
   }
 }
 
-// out[c] = sum_p partial[p * stride + c]   (p < nparts).  A CTA of 256 threads owns 32 columns: thread (cx, ry) adds up
-// rows ry, ry + 8, ... of column cx (four independent loads in flight, 128 contiguous bytes per warp and row), and the
-// eight row slices meet in shared memory.  One thread per column walking all rows, the earlier form, took as long as
-// half the norm-backward kernel that produces the partial sums.
-template <typename T>
-__global__ void reduce_partials_kernel(const float* __restrict__ partial, T* __restrict__ out, int nparts, int cols,
-                                       size_t stride) {
-  __shared__ float red[8][33];
+// out[c] = sum_p partial[p * stride + c]   (p < nparts); with gridDim.y == 2 the second row of CTAs does the same for
+// partial + H -> out2 (one launch for both sums of a LayerNorm).  A CTA owns 32 columns: thread (cx, ry) adds up
+// rows ry, ry + R, ... of column cx (four independent loads in flight, 128 contiguous bytes per warp and row), and the
+// R row slices meet in shared memory.  R is 32 where there are enough rows: the time is that of one thread's chain of
+// loads, 4.3 us for 296 rows in 8 slices.
+template <typename T, int R>
+__global__ void __launch_bounds__(32 * R) reduce_partials_kernel(const float* __restrict__ partial, T* __restrict__ out, T* __restrict__ out2,
+                                                                 int nparts, int cols, size_t stride) {
+  __shared__ float red[R][33];
   const int cx = threadIdx.x & 31, ry = threadIdx.x >> 5;
   const int c = blockIdx.x * 32 + cx;
+  if (blockIdx.y) { partial += cols; out = out2; }
   float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
   if (c < cols) {
     int p = ry;
-    for (; p + 24 < nparts; p += 32) {
+    for (; p + 3 * R < nparts; p += 4 * R) {
       a0 += partial[size_t(p) * stride + c];
-      a1 += partial[size_t(p + 8) * stride + c];
-      a2 += partial[size_t(p + 16) * stride + c];
-      a3 += partial[size_t(p + 24) * stride + c];
+      a1 += partial[size_t(p + R) * stride + c];
+      a2 += partial[size_t(p + 2 * R) * stride + c];
+      a3 += partial[size_t(p + 3 * R) * stride + c];
     }
-    for (; p < nparts; p += 8) a0 += partial[size_t(p) * stride + c];
+    for (; p < nparts; p += R) a0 += partial[size_t(p) * stride + c];
   }
   red[ry][cx] = (a0 + a1) + (a2 + a3);
   __syncthreads();
   if (ry == 0 && c < cols) {
     float acc = 0.f;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) acc += red[i][cx];
+    for (int i = 0; i < R; ++i) acc += red[i][cx];
     out[c] = from_f<T>(acc);
   }
+}
+template <typename T>
+static void reduce_partials(const float* partial, T* out, T* out2, int nparts, int cols, size_t stride, cudaStream_t stream) {
+  const dim3 grid((cols + 31) / 32, out2 ? 2 : 1);
+  if (nparts >= 128) reduce_partials_kernel<T, 32><<<grid, 1024, 0, stream>>>(partial, out, out2, nparts, cols, stride);
+  else reduce_partials_kernel<T, 8><<<grid, 256, 0, stream>>>(partial, out, out2, nparts, cols, stride);
 }
 
 // ---------------------------------------------------------------------------------------------------------
@@ -725,10 +733,21 @@ JPB_API int jpb_norm_fwd(int layer, int dt, const void* x, const void* w, const 
   });
 }
 
-// Number of fp32 scratch elements jpb_norm_bwd needs for a given shape.
+// CTAs of the norm backward: enough to keep about 1024 threads per SM (a row of 1600 bf16 is a CTA of 128 threads, and
+// two of those per SM left the memory system idle most of the time: 16384 rows took 121 us), but eight rows or more
+// each beyond two per SM, since every CTA leaves 2 H partial sums behind.
+static int norm_bwd_grid(int rows, int H, int vn) {
+  const int threads = norm_threads(H, vn, NORM_BWD_VECS);
+  const int per_sm = threads >= 512 ? 2 : 1024 / threads < 8 ? 1024 / threads : 8;
+  int grid = sm_count() * 2;
+  if (rows / 8 > grid) grid = rows / 8 < sm_count() * per_sm ? rows / 8 : sm_count() * per_sm;
+  return rows < grid ? rows : grid;
+}
+
+// Number of fp32 scratch elements jpb_norm_bwd needs for a given shape (of either type).
 JPB_API long long jpb_norm_bwd_scratch_elems(int rows, int H) {
-  const int grid = rows < sm_count() * 2 ? rows : sm_count() * 2;
-  return (long long)grid * 2 * H;
+  const int a = norm_bwd_grid(rows, H, Vec<float>::N), b = norm_bwd_grid(rows, H, Vec<__nv_bfloat16>::N);
+  return (long long)(a > b ? a : b) * 2 * H;
 }
 
 static int norm_bwd_impl(int layer, int dt, const void* dy, const void* x, const void* w, const float* mean,
@@ -739,7 +758,7 @@ static int norm_bwd_impl(int layer, int dt, const void* dy, const void* x, const
     constexpr int VN = Vec<T>::N;
     if (H % VN || H / VN > NORM_BWD_VECS * 1024) return -int(JPB_ERR_BAD_ARGUMENT);
     const int threads = norm_threads(H, VN, NORM_BWD_VECS);
-    const int grid = rows < sm_count() * 2 ? rows : sm_count() * 2;
+    const int grid = norm_bwd_grid(rows, H, VN);
     if (threads > 512) {
       if (layer)
         norm_bwd_kernel<T, true, 1024><<<grid, threads, 0, STREAM>>>((const T*)dy, (const T*)x, (const T*)w, mean, rstd, (T*)dx, scratch, rows, H, (const T*)add);
@@ -750,8 +769,7 @@ static int norm_bwd_impl(int layer, int dt, const void* dy, const void* x, const
     } else {
       norm_bwd_kernel<T, false><<<grid, threads, 0, STREAM>>>((const T*)dy, (const T*)x, (const T*)w, nullptr, rstd, (T*)dx, scratch, rows, H, (const T*)add);
     }
-    reduce_partials_kernel<T><<<(H + 31) / 32, 256, 0, STREAM>>>(scratch, (T*)dw, grid, H, size_t(2) * H);
-    if (layer) reduce_partials_kernel<T><<<(H + 31) / 32, 256, 0, STREAM>>>(scratch + H, (T*)db, grid, H, size_t(2) * H);
+    reduce_partials<T>(scratch, (T*)dw, layer ? (T*)db : nullptr, grid, H, size_t(2) * H, STREAM);
     return LAST_ERR;
   });
 }
@@ -782,7 +800,7 @@ JPB_API int jpb_colsum(int dt, const void* x, void* out, float* scratch, int row
     const int threads = 128;
     dim3 grid((cols / VN + threads - 1) / threads, parts);
     colsum_partial_kernel<T><<<grid, threads, 0, STREAM>>>((const T*)x, scratch, rows, cols);
-    reduce_partials_kernel<T><<<(cols + 31) / 32, 256, 0, STREAM>>>(scratch, (T*)out, parts, cols, size_t(cols));
+    reduce_partials<T>(scratch, (T*)out, nullptr, parts, cols, size_t(cols), STREAM);
     return LAST_ERR;
   });
 }
@@ -991,7 +1009,7 @@ JPB_API int jpb_rmsnorm_bwd_noalloc(int dtype, const void* dy, const void* x, co
     else
       norm_bwd_kernel<T, false><<<grid, threads, 0, STREAM>>>((const T*)dy, (const T*)x, (const T*)w, nullptr, rstd, (T*)dx,
                                                               scratch, rows, H);
-    reduce_partials_kernel<T><<<(H + 31) / 32, 256, 0, STREAM>>>(scratch, (T*)dw, grid, H, size_t(2) * H);
+    reduce_partials<T>(scratch, (T*)dw, nullptr, grid, H, size_t(2) * H, STREAM);
     return LAST_ERR;
   });
 }

@@ -335,7 +335,7 @@ def _norm_bwd_add(layer, dy, x, w, mean, rstd, add):
     scratch = norm_bwd_scratch(rows, H, x.device)
     _check(lib.jpb_norm_bwd_add(layer, _dt(x), dy.data_ptr(), x.data_ptr(), w.data_ptr(), _p(mean), rstd.data_ptr(),
                                 dx.data_ptr(), dw.data_ptr(), _p(db), scratch.data_ptr(), rows, H, add.data_ptr(), _stream()),
-           "norm_bwd_add", 3 if layer else 2)
+           "norm_bwd_add", 2)
     return (dx, dw, db) if layer else (dx, dw)
 
 
@@ -364,7 +364,7 @@ def layernorm_bwd(dy, x, w, mean, rstd):
     scratch = norm_bwd_scratch(rows, H, x.device)
     _check(load().jpb_norm_bwd(1, _dt(x), dy.data_ptr(), x.data_ptr(), w.data_ptr(), mean.data_ptr(), rstd.data_ptr(),
                                dx.data_ptr(), dw.data_ptr(), db.data_ptr(), scratch.data_ptr(), rows, H, _stream()),
-           "layernorm_bwd", 3)
+           "layernorm_bwd", 2)
     return dx, dw, db
 
 
