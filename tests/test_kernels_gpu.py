@@ -316,6 +316,37 @@ def test_route_tokens_kernel_matches_the_composition(native, T, E, k, dtype):
     assert (got.double() - want).norm() <= bound * want.norm()
 
 
+@pytest.mark.parametrize("layer", [False, True])
+@pytest.mark.parametrize("rows,H", [(2400, 1600), (9500, 256), (4737, 4096), (300, 8192)])
+def test_norm_backward_over_many_rows(native, layer, rows, H):
+    """More CTAs than two per SM, CTAs with unequal numbers of rows: against 64 bits, everything rounded once to bf16
+    (2^-9) after fp32 arithmetic."""
+    x, w, dy = rnd(rows, H, seed=1), rnd(H, seed=2), rnd(rows, H, seed=3)
+    xd, g = x.double(), dy.double() * w.double()
+    mean = xd.mean(-1, keepdim=True) if layer else torch.zeros(rows, 1, dtype=torch.float64, device="cuda")
+    rstd = ((xd - mean).pow(2).mean(-1, keepdim=True) + 1e-5).rsqrt()
+    xh = (xd - mean) * rstd
+    want = [(g - (g.mean(-1, keepdim=True) if layer else 0) - xh * (g * xh).mean(-1, keepdim=True)) * rstd, (dy.double() * xh).sum(0)]
+    m, r = mean.float().reshape(-1), rstd.float().reshape(-1)
+    got = native.layernorm_bwd(dy, x, w, m, r) if layer else native.rmsnorm_bwd(dy, x, w, r)
+    if layer:
+        want.append(dy.double().sum(0))
+    for a, b in zip(got, want):
+        assert (a.double() - b).norm() <= 2.0 ** -8 * b.norm()
+
+
+def test_embedding_gradient_into_any_accumulator(native):
+    """Repeated tokens, and an accumulator that does not start on a 16-byte boundary (no vector reductions there)."""
+    ids = torch.randint(0, 7, (500,), generator=torch.Generator().manual_seed(2)).cuda()
+    dy = rnd(500, 24, seed=5)
+    want = torch.zeros(7, 24, dtype=torch.float64, device="cuda").index_add_(0, ids, dy.double())
+    slack = 500 * 2.0 ** -23 * torch.zeros_like(want).index_add_(0, ids, dy.double().abs())
+    for offset in (0, 1):
+        acc = torch.ones(7 * 24 + 4, device="cuda")[offset:offset + 7 * 24].view(7, 24)
+        native.embedding_bwd(dy, ids, 7, torch.float32, out=acc, accumulate=True)
+        assert ((acc.double() - 1 - want).abs() <= slack + 2.0 ** -20).all()
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_dropout_matches_counter_based_reference(native, dtype):
     from jaxpp_b200.ops import core as ops
