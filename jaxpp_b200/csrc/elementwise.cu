@@ -673,23 +673,104 @@ __global__ void ce_bwd_kernel(const float* __restrict__ dloss, const T* __restri
 // ---------------------------------------------------------------------------------------------------------
 // AdamW: fp32 master/m/v, gradient of type G, writes new state and a low-precision copy of type O
 // ---------------------------------------------------------------------------------------------------------
-template <typename G, typename O>
+// Four consecutive elements of G / O, 8 or 16 bytes.
+template <typename T> __device__ __forceinline__ void load4(const T* p, float (&f)[4]);
+template <> __device__ __forceinline__ void load4<float>(const float* p, float (&f)[4]) {
+  const float4 v = *reinterpret_cast<const float4*>(p);
+  f[0] = v.x; f[1] = v.y; f[2] = v.z; f[3] = v.w;
+}
+template <> __device__ __forceinline__ void load4<__nv_bfloat16>(const __nv_bfloat16* p, float (&f)[4]) {
+  const uint2 v = *reinterpret_cast<const uint2*>(p);
+  const float2 a = unpack_bf16(v.x), b = unpack_bf16(v.y);
+  f[0] = a.x; f[1] = a.y; f[2] = b.x; f[3] = b.y;
+}
+__device__ __forceinline__ void store4(float* p, const float (&f)[4]) { *reinterpret_cast<float4*>(p) = make_float4(f[0], f[1], f[2], f[3]); }
+__device__ __forceinline__ void store4(__nv_bfloat16* p, const float (&f)[4]) {
+  *reinterpret_cast<uint2*>(p) = make_uint2(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]));
+}
+
+// `clip` (optional, one value on the device) scales the gradient: the global-norm clipping coefficient.  V elements per
+// thread and step: 4 where every pointer allows it.
+template <typename G, typename O, int V>
 __global__ void adamw_kernel(const float* __restrict__ p, const G* __restrict__ g, const float* __restrict__ m,
-                             const float* __restrict__ v, const int64_t* __restrict__ step, float* __restrict__ p_out,
-                             float* __restrict__ m_out, float* __restrict__ v_out, O* __restrict__ lp_out, size_t n, float lr,
-                             float beta1, float beta2, float eps, float wd, float gscale) {
+                             const float* __restrict__ v, const int64_t* __restrict__ step, const float* __restrict__ clip,
+                             float* __restrict__ p_out, float* __restrict__ m_out, float* __restrict__ v_out,
+                             O* __restrict__ lp_out, size_t n, float lr, float beta1, float beta2, float eps, float wd,
+                             float gscale) {
   const float t = float(*step);
   const float bc1 = 1.f - powf(beta1, t);
   const float bc2 = 1.f - powf(beta2, t);
-  for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += size_t(gridDim.x) * blockDim.x) {
-    const float gi = to_f(g[i]) * gscale;
-    const float mi = beta1 * m[i] + (1.f - beta1) * gi;
-    const float vi = beta2 * v[i] + (1.f - beta2) * gi * gi;
+  const float c = clip ? *clip : 1.f;
+  auto one = [&](float pi, float gi, float& mi, float& vi) {
+    gi = gi * c * gscale;
+    mi = beta1 * mi + (1.f - beta1) * gi;
+    vi = beta2 * vi + (1.f - beta2) * gi * gi;
     const float upd = (mi / bc1) / (sqrtf(vi / bc2) + eps);
-    const float pi = p[i] * (1.f - lr * wd) - lr * upd;
+    return pi * (1.f - lr * wd) - lr * upd;
+  };
+  const size_t first = size_t(blockIdx.x) * blockDim.x + threadIdx.x, stride = size_t(gridDim.x) * blockDim.x;
+  size_t done = 0;
+  if constexpr (V == 4) {
+    done = n & ~size_t(3);
+    for (size_t i = first * 4; i < done; i += stride * 4) {
+      float pf[4], gf[4], mf[4], vf[4];
+      load4(p + i, pf); load4(g + i, gf); load4(m + i, mf); load4(v + i, vf);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) pf[j] = one(pf[j], gf[j], mf[j], vf[j]);
+      store4(p_out + i, pf); store4(m_out + i, mf); store4(v_out + i, vf); store4(lp_out + i, pf);
+    }
+  }
+  for (size_t i = done + first; i < n; i += stride) {
+    float mi = m[i], vi = v[i];
+    const float pi = one(p[i], to_f(g[i]), mi, vi);
     p_out[i] = pi; m_out[i] = mi; v_out[i] = vi;
     lp_out[i] = from_f<O>(pi);
   }
+}
+
+// ---------------------------------------------------------------------------------------------------------
+// Sum of squares over several tensors (a global gradient norm): every CTA takes SQ_CHUNK elements of one tensor and
+// leaves one partial sum, a second kernel adds the partial sums in a fixed order.  One read of the data and two launches
+// for up to SQ_TENSORS tensors, where square, sum and running total were three or four launches and five passes each.
+// ---------------------------------------------------------------------------------------------------------
+constexpr int SQ_TENSORS = 48, SQ_CHUNK = 32768, SQ_THREADS = 256;
+struct SqArgs {
+  const void* ptr[SQ_TENSORS];
+  long long size[SQ_TENSORS];
+  int first[SQ_TENSORS + 1];   // first CTA of each tensor
+  int count;
+};
+
+template <typename T>
+__global__ void __launch_bounds__(SQ_THREADS) sum_squares_kernel(const __grid_constant__ SqArgs a, float* __restrict__ partial) {
+  constexpr int VN = Vec<T>::N;
+  __shared__ float scratch[32];
+  int t = 0;
+  while (t + 1 < a.count && int(blockIdx.x) >= a.first[t + 1]) ++t;
+  const T* x = static_cast<const T*>(a.ptr[t]);
+  const long long begin = (long long)(int(blockIdx.x) - a.first[t]) * SQ_CHUNK;
+  const int n = int(a.size[t] - begin < SQ_CHUNK ? a.size[t] - begin : SQ_CHUNK);
+  x += begin;
+  float acc[4] = {0.f, 0.f, 0.f, 0.f};
+  const int vecs = (reinterpret_cast<uintptr_t>(x) & 15) == 0 ? n / VN : 0;
+  for (int v = threadIdx.x; v < vecs; v += SQ_THREADS) {
+    Vec<T> xv; xv.load(x + v * VN);
+    float f[VN]; xv.to_float(f);
+#pragma unroll
+    for (int j = 0; j < VN; ++j) acc[j & 3] += f[j] * f[j];
+  }
+  for (int i = vecs * VN + threadIdx.x; i < n; i += SQ_THREADS) { const float f = to_f(x[i]); acc[0] += f * f; }
+  float s[1] = {(acc[0] + acc[1]) + (acc[2] + acc[3])};
+  block_sum<1>(s, scratch);
+  if (threadIdx.x == 0) partial[blockIdx.x] = s[0];
+}
+
+__global__ void __launch_bounds__(1024) sum_partials_kernel(const float* __restrict__ partial, int n, float* __restrict__ out) {
+  __shared__ float scratch[32];
+  float s[1] = {0.f};
+  for (int i = threadIdx.x; i < n; i += 1024) s[0] += partial[i];
+  block_sum<1>(s, scratch);
+  if (threadIdx.x == 0) *out = s[0];
 }
 
 static int sm_count() {
@@ -950,13 +1031,50 @@ JPB_API int jpb_ce_bwd(int dt, const float* dloss, const void* logits, const lon
   });
 }
 
+// CTAs that jpb_sum_squares_partial launches for a tensor of n elements = partial sums that it writes.
+JPB_API long long jpb_sum_squares_parts(long long n) { return (n + SQ_CHUNK - 1) / SQ_CHUNK; }
+
+// One partial sum of squares per chunk of each of `count` contiguous tensors of one type, in order.
+JPB_API int jpb_sum_squares_partial(int dt, int count, const void* const* ptrs, const long long* sizes, float* partial, void* stream) {
+  return dispatch_dtype(dt, [&](auto tag) {
+    using T = decltype(tag);
+    for (int base = 0; base < count; base += SQ_TENSORS) {
+      SqArgs a;
+      a.count = count - base < SQ_TENSORS ? count - base : SQ_TENSORS;
+      long long blocks = 0;
+      for (int i = 0; i < a.count; ++i) {
+        a.ptr[i] = ptrs[base + i];
+        a.size[i] = sizes[base + i];
+        a.first[i] = int(blocks);
+        blocks += jpb_sum_squares_parts(sizes[base + i]);
+      }
+      if (blocks > 0x7fffffffll) return -int(JPB_ERR_BAD_ARGUMENT);
+      if (blocks > 0) sum_squares_kernel<T><<<unsigned(blocks), SQ_THREADS, 0, STREAM>>>(a, partial);
+      partial += blocks;
+    }
+    return LAST_ERR;
+  });
+}
+
+JPB_API int jpb_sum_partials(const float* partial, int n, float* out, void* stream) {
+  sum_partials_kernel<<<1, 1024, 0, STREAM>>>(partial, n, out);
+  return LAST_ERR;
+}
+
 JPB_API int jpb_adamw(int grad_dt, int out_dt, const float* p, const void* g, const float* m, const float* v,
-                      const long long* step, float* p_out, float* m_out, float* v_out, void* lp_out, long long n, float lr,
-                      float beta1, float beta2, float eps, float wd, float gscale, void* stream) {
-  const int grid = ew_grid(size_t(n), 256);
-#define ADAMW(G, O)                                                                                                      \
-  adamw_kernel<G, O><<<grid, 256, 0, STREAM>>>(p, (const G*)g, m, v, (const int64_t*)step, p_out, m_out, v_out, (O*)lp_out, \
-                                               size_t(n), lr, beta1, beta2, eps, wd, gscale)
+                      const long long* step, const float* clip, float* p_out, float* m_out, float* v_out, void* lp_out, long long n,
+                      float lr, float beta1, float beta2, float eps, float wd, float gscale, void* stream) {
+  uintptr_t at = 0;   // (16-byte alignment is more than a bf16 gradient or copy needs, and is what allocations have)
+  for (const void* x : {(const void*)p, g, (const void*)m, (const void*)v, (const void*)p_out, (const void*)m_out, (const void*)v_out,
+                        (const void*)lp_out})
+    at |= reinterpret_cast<uintptr_t>(x);
+  const bool wide = (at & 15) == 0;
+  const int grid = ew_grid(wide ? size_t(n + 3) / 4 : size_t(n), 256);
+#define ADAMW(G, O)                                                                                                                \
+  (wide ? adamw_kernel<G, O, 4><<<grid, 256, 0, STREAM>>>(p, (const G*)g, m, v, (const int64_t*)step, clip, p_out, m_out, v_out,    \
+                                                          (O*)lp_out, size_t(n), lr, beta1, beta2, eps, wd, gscale)                \
+        : adamw_kernel<G, O, 1><<<grid, 256, 0, STREAM>>>(p, (const G*)g, m, v, (const int64_t*)step, clip, p_out, m_out, v_out,    \
+                                                          (O*)lp_out, size_t(n), lr, beta1, beta2, eps, wd, gscale))
   if (grad_dt == 0 && out_dt == 0) ADAMW(float, float);
   else if (grad_dt == 0 && out_dt == 1) ADAMW(float, __nv_bfloat16);
   else if (grad_dt == 1 && out_dt == 0) ADAMW(__nv_bfloat16, float);

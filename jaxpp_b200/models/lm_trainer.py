@@ -166,17 +166,15 @@ def make_train_step(cfg: tf.ModelConfig, schedule, hyper: Hyper = Hyper(), dp_ax
                                      hyper.clip_grad_norm, 1.0 / total_tokens)
 
         def update(p, master, g, m, v, keep_whole=True):
-            if clip is not None:
-                g = g * clip.to(g.dtype)
             if not keep_whole:
                 # AdamW on the slice -> bf16 slice -> parameter gathered from the owners of the slices
                 pm, mm, vm, lp = ops.adamw(master, g, m, v, new_step, hyper.lr, hyper.beta1, hyper.beta2, hyper.eps,
                                            hyper.weight_decay if p.dim() > 1 else 0.0, 1.0 / total_tokens, p.dtype,
-                                           None, hyper.inplace_update)
+                                           None, hyper.inplace_update, clip)
                 return zero.all_gather_flat(lp, dp_axis, p.numel()).view(p.shape), pm, mm, vm
             pm, mm, vm, lp = ops.adamw(master, g, m, v, new_step, hyper.lr, hyper.beta1, hyper.beta2, hyper.eps,
                                        hyper.weight_decay if p.dim() > 1 else 0.0, 1.0 / total_tokens, p.dtype,
-                                       p if hyper.inplace_update else None, hyper.inplace_update)
+                                       p if hyper.inplace_update else None, hyper.inplace_update, clip)
             return lp, pm, mm, vm
 
         flat = [update(p, ma, g, m, v, k) for p, ma, g, m, v, k in zip(
@@ -210,7 +208,7 @@ def _clip_coefficient(cfg: tf.ModelConfig, schedule, params: dict, flat_g: list,
         else:
             paths.append((owners["embed" if k in ("embed", "pos") else "head"], k))
     assert len(paths) == len(flat_g)
-    groups: dict = {}  # (rank, axes to complete over) -> sum of squares
+    groups: dict = {}  # (rank, axes to complete over) -> gradients
     for (rank, name), g, keep_whole in zip(paths, flat_g, whole):
         axes = []
         if name in tp_sharded:
@@ -219,11 +217,10 @@ def _clip_coefficient(cfg: tf.ModelConfig, schedule, params: dict, flat_g: list,
             axes.append(cfg.ep_axis)
         elif not keep_whole:
             axes.append(dp_axis)      # a 1/dp slice of a replicated parameter's gradient
-        sq = g.float().pow(2).sum()
-        key = (rank, tuple(dict.fromkeys(axes)))
-        groups[key] = sq if key not in groups else groups[key] + sq
+        groups.setdefault((rank, tuple(dict.fromkeys(axes))), []).append(g)
     per_rank: dict = {}
-    for (rank, axes), sq in groups.items():
+    for (rank, axes), gs in groups.items():
+        sq = ops.sum_squares(gs)
         for axis in axes:
             sq = tpops.all_reduce(sq.reshape(1), axis).reshape(())
         per_rank[rank] = sq if rank not in per_rank else per_rank[rank] + sq

@@ -734,9 +734,25 @@ _autograd("embedding",
 # ``master``/``m``/``v`` are fp32; ``grad`` may be bf16 or fp32; ``step`` is a 0-d tensor (1-based)
 # ======================================================================================
 
+def _sum_squares_impl(tensors):
+    if _use_native(tensors[0]) and all(t.device == tensors[0].device and t.dtype in (torch.float32, torch.bfloat16) for t in tensors):
+        return _native().sum_squares(tensors)
+    total = _f32(tensors[0]).pow(2).sum()
+    for t in tensors[1:]:
+        total = total + _f32(t).pow(2).sum()
+    return total
+
+
+_lib.define("sum_squares(Tensor[] tensors) -> Tensor")
+_lib.impl("sum_squares", _sum_squares_impl, "CompositeExplicitAutograd")
+torch.library.register_fake("b200::sum_squares", lambda tensors: tensors[0].new_empty((), dtype=torch.float32))
+sum_squares = torch.ops.b200.sum_squares
+DIRECT[sum_squares.default] = _sum_squares_impl
+
+
 def _adamw_ref(master, grad, m, v, step, lr, beta1, beta2, eps, weight_decay, grad_scale, out_dtype, lp_old=None,
-               inplace=False):
-    g = _f32(grad) * grad_scale
+               inplace=False, clip=None):
+    g = (_f32(grad) if clip is None else _f32(grad) * clip) * grad_scale
     m2 = beta1 * m + (1.0 - beta1) * g
     v2 = beta2 * v + (1.0 - beta2) * g * g
     t = step.to(torch.float32)
@@ -753,10 +769,10 @@ def _adamw_ref(master, grad, m, v, step, lr, beta1, beta2, eps, weight_decay, gr
 
 adamw = _define(
     "adamw(Tensor master, Tensor grad, Tensor m, Tensor v, Tensor step, float lr, float beta1, float beta2,"
-    " float eps, float weight_decay, float grad_scale, ScalarType out_dtype, Tensor? lp_old=None, bool inplace=False)"
-    " -> (Tensor, Tensor, Tensor, Tensor)",
+    " float eps, float weight_decay, float grad_scale, ScalarType out_dtype, Tensor? lp_old=None, bool inplace=False,"
+    " Tensor? clip=None) -> (Tensor, Tensor, Tensor, Tensor)",
     _adamw_ref,
-    lambda master, grad, m, v, step, lr, b1, b2, eps, wd, gs, out_dtype, lp_old=None, inplace=False: (
+    lambda master, grad, m, v, step, lr, b1, b2, eps, wd, gs, out_dtype, lp_old=None, inplace=False, clip=None: (
         torch.empty_like(master),
         torch.empty_like(m),
         torch.empty_like(v),
@@ -777,5 +793,5 @@ def mse_loss(out: Tensor, target: Tensor) -> Tensor:
 __all__ = [
     "linear", "linear_dgrad", "linear_wgrad", "colsum", "rmsnorm", "rmsnorm_bwd", "layernorm", "layernorm_bwd",
     "gelu", "gelu_bwd", "swiglu", "swiglu_bwd", "rope", "attention", "attention_bwd", "cross_entropy",
-    "cross_entropy_bwd", "embedding", "embedding_bwd", "adamw", "mse_loss",
+    "cross_entropy_bwd", "embedding", "embedding_bwd", "sum_squares", "adamw", "mse_loss",
 ]

@@ -52,7 +52,11 @@ def load() -> ctypes.CDLL:
     lib.jpb_embedding_bwd.argtypes = [_c_int, _c_p, _c_p, _c_p, _c_p, _c_ll, _c_int, _c_int, _c_p]
     lib.jpb_ce_fwd.argtypes = [_c_int, _c_p, _c_p, _c_p, _c_p, _c_int, _c_int, _c_p]
     lib.jpb_ce_bwd.argtypes = [_c_int, _c_p, _c_p, _c_p, _c_p, _c_p, _c_int, _c_int, _c_p]
-    lib.jpb_adamw.argtypes = [_c_int, _c_int] + [_c_p] * 9 + [_c_ll] + [_c_f] * 6 + [_c_p]
+    lib.jpb_adamw.argtypes = [_c_int, _c_int] + [_c_p] * 10 + [_c_ll] + [_c_f] * 6 + [_c_p]
+    lib.jpb_sum_squares_parts.argtypes = [_c_ll]
+    lib.jpb_sum_squares_parts.restype = _c_ll
+    lib.jpb_sum_squares_partial.argtypes = [_c_int, _c_int, _c_p, _c_p, _c_p, _c_p]
+    lib.jpb_sum_partials.argtypes = [_c_p, _c_int, _c_p, _c_p]
     lib.jpb_read_status.argtypes = [_c_int]
     lib.jpb_build_info.restype = ctypes.c_char_p
     for name in ("jpb_attention_fwd", "jpb_attention_bwd"):
@@ -509,9 +513,31 @@ def cross_entropy_bwd(dloss, logits, labels, lse):
     return out
 
 
+def sum_squares(tensors):
+    """Sum of the squares of all elements of float32 / bfloat16 tensors, as one float32 value on their device."""
+    lib = load()
+    by_type: dict = {}
+    for t in tensors:
+        by_type.setdefault(_dt(t), []).append(t.contiguous())
+    parts = {dt: sum(lib.jpb_sum_squares_parts(t.numel()) for t in ts) for dt, ts in by_type.items()}
+    device = tensors[0].device
+    partial = torch.empty(max(1, sum(parts.values())), dtype=torch.float32, device=device)
+    out = torch.empty((), dtype=torch.float32, device=device)
+    at = 0
+    for dt, ts in by_type.items():
+        ptrs = (ctypes.c_void_p * len(ts))(*[t.data_ptr() for t in ts])
+        sizes = (_c_ll * len(ts))(*[t.numel() for t in ts])
+        _check(lib.jpb_sum_squares_partial(dt, len(ts), ptrs, sizes, partial.data_ptr() + 4 * at, _stream()), "sum_squares")
+        at += parts[dt]
+    _check(lib.jpb_sum_partials(partial.data_ptr(), at, out.data_ptr(), _stream()), "sum_partials")
+    return out
+
+
 def adamw(master, grad, m, v, step, lr, beta1, beta2, eps, weight_decay, grad_scale, out_dtype, lp_old=None,
-          inplace=False):
+          inplace=False, clip=None):
     grad = grad.contiguous()
+    if clip is not None:
+        clip = clip.to(device=master.device, dtype=torch.float32)
     if inplace:
         if not (master.is_contiguous() and m.is_contiguous() and v.is_contiguous()):
             raise NativeError("in-place adamw needs contiguous state tensors")
@@ -527,7 +553,7 @@ def adamw(master, grad, m, v, step, lr, beta1, beta2, eps, weight_decay, grad_sc
     if out_dtype not in (torch.float32, torch.bfloat16):
         raise NativeError(f"adamw low-precision copy must be float32 or bfloat16, got {out_dtype}")
     _check(load().jpb_adamw(_dt(grad), out_code, master.data_ptr(), grad.data_ptr(), m.data_ptr(), v.data_ptr(),
-                            step.data_ptr(), p2.data_ptr(), m2.data_ptr(), v2.data_ptr(), lp.data_ptr(), master.numel(),
+                            step.data_ptr(), _p(clip), p2.data_ptr(), m2.data_ptr(), v2.data_ptr(), lp.data_ptr(), master.numel(),
                             float(lr), float(beta1), float(beta2), float(eps), float(weight_decay), float(grad_scale),
                             _stream()), "adamw")
     return p2, m2, v2, lp

@@ -347,6 +347,33 @@ def test_embedding_gradient_into_any_accumulator(native):
         assert ((acc.double() - 1 - want).abs() <= slack + 2.0 ** -20).all()
 
 
+def test_sum_squares_over_many_tensors(native):
+    """More tensors than one launch takes, of both types, single elements, chunk edges and an unaligned view."""
+    ts = [rnd(n, dtype=dt, seed=n) for n in (1, 3, 32768, 32769, 100003) for dt in (torch.float32, torch.bfloat16)]
+    ts += [rnd(1000, dtype=torch.float32, seed=7)[1:]] + [rnd(10 + i, dtype=torch.float32, seed=i) for i in range(50)]
+    want = sum(t.double().pow(2).sum() for t in ts)
+    assert abs(native.sum_squares(ts).double() - want) <= 1e-5 * want   # chains of fewer than 160 fp32 additions
+
+
+@pytest.mark.parametrize("n,offset", [(1, 0), (3, 0), (1027, 0), (4096, 0), (1026, 1)])
+@pytest.mark.parametrize("gdt", [torch.float32, torch.bfloat16])
+def test_adamw_with_clip_coefficient(native, n, offset, gdt):
+    """Whole and partial vectors, unaligned state, the clipping coefficient as a value on the device, in place or not."""
+    from jaxpp_b200.ops import core as ops
+
+    make = lambda seed: rnd(n + offset, dtype=torch.float32, seed=seed)[offset:]
+    p, m, v, g = make(1), make(2), make(3).abs(), make(4).to(gdt)
+    step, clip = torch.tensor(7, device="cuda"), torch.tensor(0.37, device="cuda")
+    for c in (clip, None):
+        args = (step, 1e-2, 0.9, 0.95, 1e-8, 0.1, 0.5, torch.bfloat16)
+        want = ops._adamw_ref(p.double(), g.double(), m.double(), v.double(), *args, None, False, c)
+        state = [t.clone() for t in (p, m, v)]
+        got = native.adamw(state[0], g, state[1], state[2], *args, None, offset == 0, c)
+        for a, b in zip(got[:3], want[:3]):
+            close(a, b.float(), rtol=1e-5, atol=1e-6)
+        assert torch.equal(got[3], got[0].to(torch.bfloat16))
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_dropout_matches_counter_based_reference(native, dtype):
     from jaxpp_b200.ops import core as ops
