@@ -138,6 +138,9 @@ class Lowering:
             from .peephole import fuse_norm_backward_adds
 
             fuse_norm_backward_adds(graph)
+        from .peephole import widen_parameter_sums
+
+        widen_parameter_sums(graph, keep={o for o in cap.outputs if isinstance(o, fx.Node)})
         loop = cl.find_loop(graph)
         nodes = list(graph.nodes)
         self.pos = {n: i for i, n in enumerate(nodes)}

@@ -271,10 +271,10 @@ __global__ void __launch_bounds__(MAXT) norm_bwd_kernel(const T* __restrict__ dy
 // partial + H -> out2 (one launch for both sums of a LayerNorm).  A CTA owns 32 columns: thread (cx, ry) adds up
 // rows ry, ry + R, ... of column cx (four independent loads in flight, 128 contiguous bytes per warp and row), and the
 // R row slices meet in shared memory.  R is 32 where there are enough rows: the time is that of one thread's chain of
-// loads, 4.3 us for 296 rows in 8 slices.
+// loads, 4.3 us for 296 rows in 8 slices.  The sums leave as T or, with `wide`, in fp32.
 template <typename T, int R>
-__global__ void __launch_bounds__(32 * R) reduce_partials_kernel(const float* __restrict__ partial, T* __restrict__ out, T* __restrict__ out2,
-                                                                 int nparts, int cols, size_t stride) {
+__global__ void __launch_bounds__(32 * R) reduce_partials_kernel(const float* __restrict__ partial, void* __restrict__ out, void* __restrict__ out2,
+                                                                 int nparts, int cols, size_t stride, int wide) {
   __shared__ float red[R][33];
   const int cx = threadIdx.x & 31, ry = threadIdx.x >> 5;
   const int c = blockIdx.x * 32 + cx;
@@ -296,14 +296,15 @@ __global__ void __launch_bounds__(32 * R) reduce_partials_kernel(const float* __
     float acc = 0.f;
 #pragma unroll
     for (int i = 0; i < R; ++i) acc += red[i][cx];
-    out[c] = from_f<T>(acc);
+    if (wide) static_cast<float*>(out)[c] = acc;
+    else static_cast<T*>(out)[c] = from_f<T>(acc);
   }
 }
 template <typename T>
-static void reduce_partials(const float* partial, T* out, T* out2, int nparts, int cols, size_t stride, cudaStream_t stream) {
+static void reduce_partials(const float* partial, void* out, void* out2, int nparts, int cols, size_t stride, int wide, cudaStream_t stream) {
   const dim3 grid((cols + 31) / 32, out2 ? 2 : 1);
-  if (nparts >= 128) reduce_partials_kernel<T, 32><<<grid, 1024, 0, stream>>>(partial, out, out2, nparts, cols, stride);
-  else reduce_partials_kernel<T, 8><<<grid, 256, 0, stream>>>(partial, out, out2, nparts, cols, stride);
+  if (nparts >= 128) reduce_partials_kernel<T, 32><<<grid, 1024, 0, stream>>>(partial, out, out2, nparts, cols, stride, wide);
+  else reduce_partials_kernel<T, 8><<<grid, 256, 0, stream>>>(partial, out, out2, nparts, cols, stride, wide);
 }
 
 // ---------------------------------------------------------------------------------------------------------
@@ -839,7 +840,7 @@ JPB_API long long jpb_norm_bwd_scratch_elems(int rows, int H) {
 
 static int norm_bwd_impl(int layer, int dt, const void* dy, const void* x, const void* w, const float* mean,
                          const float* rstd, void* dx, void* dw, void* db, float* scratch, int rows, int H, const void* add,
-                         void* stream) {
+                         int wide, void* stream) {
   return dispatch_dtype(dt, [&](auto tag) {
     using T = decltype(tag);
     constexpr int VN = Vec<T>::N;
@@ -856,21 +857,22 @@ static int norm_bwd_impl(int layer, int dt, const void* dy, const void* x, const
     } else {
       norm_bwd_kernel<T, false><<<grid, threads, 0, STREAM>>>((const T*)dy, (const T*)x, (const T*)w, nullptr, rstd, (T*)dx, scratch, rows, H, (const T*)add);
     }
-    reduce_partials<T>(scratch, (T*)dw, layer ? (T*)db : nullptr, grid, H, size_t(2) * H, STREAM);
+    reduce_partials<T>(scratch, dw, layer ? db : nullptr, grid, H, size_t(2) * H, wide, STREAM);
     return LAST_ERR;
   });
 }
 
+// dw and db are of the type of x or, with `wide`, fp32.
 JPB_API int jpb_norm_bwd(int layer, int dt, const void* dy, const void* x, const void* w, const float* mean,
-                         const float* rstd, void* dx, void* dw, void* db, float* scratch, int rows, int H, void* stream) {
-  return norm_bwd_impl(layer, dt, dy, x, w, mean, rstd, dx, dw, db, scratch, rows, H, nullptr, stream);
+                         const float* rstd, void* dx, void* dw, void* db, float* scratch, int rows, int H, int wide, void* stream) {
+  return norm_bwd_impl(layer, dt, dy, x, w, mean, rstd, dx, dw, db, scratch, rows, H, nullptr, wide, stream);
 }
 
 // Same, with the residual-path gradient `add` (shape of dx) summed into dx in the same pass.
 JPB_API int jpb_norm_bwd_add(int layer, int dt, const void* dy, const void* x, const void* w, const float* mean,
                              const float* rstd, void* dx, void* dw, void* db, float* scratch, int rows, int H,
-                             const void* add, void* stream) {
-  return norm_bwd_impl(layer, dt, dy, x, w, mean, rstd, dx, dw, db, scratch, rows, H, add, stream);
+                             const void* add, int wide, void* stream) {
+  return norm_bwd_impl(layer, dt, dy, x, w, mean, rstd, dx, dw, db, scratch, rows, H, add, wide, stream);
 }
 
 JPB_API long long jpb_colsum_scratch_elems(int rows, int cols) {
@@ -878,7 +880,8 @@ JPB_API long long jpb_colsum_scratch_elems(int rows, int cols) {
   return (long long)parts * cols;
 }
 
-JPB_API int jpb_colsum(int dt, const void* x, void* out, float* scratch, int rows, int cols, void* stream) {
+// `out` is of the type of x or, with `wide`, fp32.
+JPB_API int jpb_colsum(int dt, const void* x, void* out, float* scratch, int rows, int cols, int wide, void* stream) {
   return dispatch_dtype(dt, [&](auto tag) {
     using T = decltype(tag);
     constexpr int VN = Vec<T>::N;
@@ -887,7 +890,7 @@ JPB_API int jpb_colsum(int dt, const void* x, void* out, float* scratch, int row
     const int threads = 128;
     dim3 grid((cols / VN + threads - 1) / threads, parts);
     colsum_partial_kernel<T><<<grid, threads, 0, STREAM>>>((const T*)x, scratch, rows, cols);
-    reduce_partials<T>(scratch, (T*)out, nullptr, parts, cols, size_t(cols), STREAM);
+    reduce_partials<T>(scratch, out, nullptr, parts, cols, size_t(cols), wide, STREAM);
     return LAST_ERR;
   });
 }
@@ -1133,7 +1136,7 @@ JPB_API int jpb_rmsnorm_bwd_noalloc(int dtype, const void* dy, const void* x, co
     else
       norm_bwd_kernel<T, false><<<grid, threads, 0, STREAM>>>((const T*)dy, (const T*)x, (const T*)w, nullptr, rstd, (T*)dx,
                                                               scratch, rows, H);
-    reduce_partials<T>(scratch, (T*)dw, nullptr, grid, H, size_t(2) * H, STREAM);
+    reduce_partials<T>(scratch, dw, nullptr, grid, H, size_t(2) * H, 0, STREAM);
     return LAST_ERR;
   });
 }

@@ -138,9 +138,9 @@ DIRECT[linear_wgrad.default] = _linear_wgrad_native_or_ref
 
 # column sums, used for bias gradients
 colsum = _define(
-    "colsum(Tensor dy) -> Tensor",
-    lambda dy: dy.reshape(-1, dy.shape[-1]).float().sum(0).to(dy.dtype),
-    lambda dy: dy.new_empty(dy.shape[-1]),
+    "colsum(Tensor dy, ScalarType? sum_dtype=None) -> Tensor",
+    lambda dy, sum_dtype=None: dy.reshape(-1, dy.shape[-1]).float().sum(0).to(sum_dtype or dy.dtype),
+    lambda dy, sum_dtype=None: dy.new_empty(dy.shape[-1], dtype=sum_dtype or dy.dtype),
     "colsum",
 )
 
@@ -233,34 +233,36 @@ rmsnorm = _define(
 )
 
 
-def _rmsnorm_bwd_ref(dy, x, w, rstd):
+# ``sum_dtype`` of the norm backwards and of ``colsum``: type of the parameter sums (default: the parameter's).  A step with
+# fp32 gradients asks for fp32 (compiler/peephole.py): no rounding to the parameter's type and no cast kernel behind it.
+def _rmsnorm_bwd_ref(dy, x, w, rstd, sum_dtype=None):
     xf, dyf, wf = _f32(x), _f32(dy), _f32(w)
     xhat = xf * rstd.unsqueeze(-1)
     g = dyf * wf
     dx = (g - xhat * (g * xhat).mean(-1, keepdim=True)) * rstd.unsqueeze(-1)
     dw = (dyf * xhat).reshape(-1, x.shape[-1]).sum(0)
-    return dx.to(x.dtype), dw.to(w.dtype)
+    return dx.to(x.dtype), dw.to(sum_dtype or w.dtype)
 
 
 rmsnorm_bwd = _define(
-    "rmsnorm_bwd(Tensor dy, Tensor x, Tensor w, Tensor rstd) -> (Tensor, Tensor)",
+    "rmsnorm_bwd(Tensor dy, Tensor x, Tensor w, Tensor rstd, ScalarType? sum_dtype=None) -> (Tensor, Tensor)",
     _rmsnorm_bwd_ref,
-    lambda dy, x, w, rstd: (torch.empty_like(x), torch.empty_like(w)),
+    lambda dy, x, w, rstd, sum_dtype=None: (torch.empty_like(x), torch.empty_like(w, dtype=sum_dtype)),
     "rmsnorm_bwd",
 )
 
 
-def _rmsnorm_bwd_add_ref(dy, x, w, rstd, add):
-    dx, dw = _rmsnorm_bwd_ref(dy, x, w, rstd)
+def _rmsnorm_bwd_add_ref(dy, x, w, rstd, add, sum_dtype=None):
+    dx, dw = _rmsnorm_bwd_ref(dy, x, w, rstd, sum_dtype)
     return dx + add, dw
 
 
 # dx + (gradient arriving over the residual connection) in the pass that produces dx; the graph rewrite in
 # compiler/peephole.py puts it in place of ``rmsnorm_bwd`` followed by ``add``
 rmsnorm_bwd_add = _define(
-    "rmsnorm_bwd_add(Tensor dy, Tensor x, Tensor w, Tensor rstd, Tensor add) -> (Tensor, Tensor)",
+    "rmsnorm_bwd_add(Tensor dy, Tensor x, Tensor w, Tensor rstd, Tensor add, ScalarType? sum_dtype=None) -> (Tensor, Tensor)",
     _rmsnorm_bwd_add_ref,
-    lambda dy, x, w, rstd, add: (torch.empty_like(x), torch.empty_like(w)),
+    lambda dy, x, w, rstd, add, sum_dtype=None: (torch.empty_like(x), torch.empty_like(w, dtype=sum_dtype)),
     "rmsnorm_bwd_add",
 )
 
@@ -300,33 +302,36 @@ layernorm = _define(
 )
 
 
-def _layernorm_bwd_ref(dy, x, w, mean, rstd):
+def _layernorm_bwd_ref(dy, x, w, mean, rstd, sum_dtype=None):
     xf, dyf, wf = _f32(x), _f32(dy), _f32(w)
     xhat = (xf - mean.unsqueeze(-1)) * rstd.unsqueeze(-1)
     g = dyf * wf
     dx = (g - g.mean(-1, keepdim=True) - xhat * (g * xhat).mean(-1, keepdim=True)) * rstd.unsqueeze(-1)
     dw = (dyf * xhat).reshape(-1, x.shape[-1]).sum(0)
     db = dyf.reshape(-1, x.shape[-1]).sum(0)
-    return dx.to(x.dtype), dw.to(w.dtype), db.to(w.dtype)
+    return dx.to(x.dtype), dw.to(sum_dtype or w.dtype), db.to(sum_dtype or w.dtype)
 
 
 layernorm_bwd = _define(
-    "layernorm_bwd(Tensor dy, Tensor x, Tensor w, Tensor mean, Tensor rstd) -> (Tensor, Tensor, Tensor)",
+    "layernorm_bwd(Tensor dy, Tensor x, Tensor w, Tensor mean, Tensor rstd, ScalarType? sum_dtype=None) -> (Tensor, Tensor, Tensor)",
     _layernorm_bwd_ref,
-    lambda dy, x, w, mean, rstd: (torch.empty_like(x), torch.empty_like(w), torch.empty_like(w)),
+    lambda dy, x, w, mean, rstd, sum_dtype=None: (torch.empty_like(x), torch.empty_like(w, dtype=sum_dtype),
+                                                  torch.empty_like(w, dtype=sum_dtype)),
     "layernorm_bwd",
 )
 
 
-def _layernorm_bwd_add_ref(dy, x, w, mean, rstd, add):
-    dx, dw, db = _layernorm_bwd_ref(dy, x, w, mean, rstd)
+def _layernorm_bwd_add_ref(dy, x, w, mean, rstd, add, sum_dtype=None):
+    dx, dw, db = _layernorm_bwd_ref(dy, x, w, mean, rstd, sum_dtype)
     return dx + add, dw, db
 
 
 layernorm_bwd_add = _define(
-    "layernorm_bwd_add(Tensor dy, Tensor x, Tensor w, Tensor mean, Tensor rstd, Tensor add) -> (Tensor, Tensor, Tensor)",
+    "layernorm_bwd_add(Tensor dy, Tensor x, Tensor w, Tensor mean, Tensor rstd, Tensor add, ScalarType? sum_dtype=None)"
+    " -> (Tensor, Tensor, Tensor)",
     _layernorm_bwd_add_ref,
-    lambda dy, x, w, mean, rstd, add: (torch.empty_like(x), torch.empty_like(w), torch.empty_like(w)),
+    lambda dy, x, w, mean, rstd, add, sum_dtype=None: (torch.empty_like(x), torch.empty_like(w, dtype=sum_dtype),
+                                                       torch.empty_like(w, dtype=sum_dtype)),
     "layernorm_bwd_add",
 )
 

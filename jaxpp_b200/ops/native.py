@@ -39,12 +39,12 @@ def load() -> ctypes.CDLL:
     lib = ctypes.CDLL(LIB_PATH)
     lib.jpb_gemm_bf16.argtypes = [_c_p, _c_p, _c_p, _c_p] + [_c_int] * 11 + [_c_p]
     lib.jpb_norm_fwd.argtypes = [_c_int, _c_int, _c_p, _c_p, _c_p, _c_p, _c_p, _c_p, _c_int, _c_int, _c_f, _c_p]
-    lib.jpb_norm_bwd.argtypes = [_c_int, _c_int] + [_c_p] * 9 + [_c_int, _c_int, _c_p]
+    lib.jpb_norm_bwd.argtypes = [_c_int, _c_int] + [_c_p] * 9 + [_c_int, _c_int, _c_int, _c_p]
     lib.jpb_norm_bwd_scratch_elems.argtypes = [_c_int, _c_int]
     lib.jpb_norm_bwd_scratch_elems.restype = _c_ll
     lib.jpb_colsum_scratch_elems.argtypes = [_c_int, _c_int]
     lib.jpb_colsum_scratch_elems.restype = _c_ll
-    lib.jpb_colsum.argtypes = [_c_int, _c_p, _c_p, _c_p, _c_int, _c_int, _c_p]
+    lib.jpb_colsum.argtypes = [_c_int, _c_p, _c_p, _c_p, _c_int, _c_int, _c_int, _c_p]
     lib.jpb_gelu.argtypes = [_c_int, _c_int, _c_p, _c_p, _c_p, _c_ll, _c_p]
     lib.jpb_swiglu.argtypes = [_c_int, _c_int, _c_p, _c_p, _c_p, _c_ll, _c_int, _c_p]
     lib.jpb_rope.argtypes = [_c_int, _c_p, _c_p, _c_p, _c_p, _c_ll, _c_int, _c_int, _c_int, _c_int, _c_p]
@@ -319,36 +319,45 @@ def norm_bwd_scratch(rows: int, H: int, device) -> torch.Tensor:
     return torch.empty(n, dtype=torch.float32, device=device)
 
 
-def rmsnorm_bwd(dy, x, w, rstd):
+def _wide(sum_dtype, t) -> int:
+    """Do the parameter sums of an op leave in float32 although its tensors are of another type?"""
+    if sum_dtype is None or sum_dtype == t.dtype:
+        return 0
+    if sum_dtype != torch.float32:
+        raise NativeError(f"parameter sums are {t.dtype} or float32, not {sum_dtype}")
+    return 1
+
+
+def rmsnorm_bwd(dy, x, w, rstd, sum_dtype=None):
     dy, x, w = dy.contiguous(), x.contiguous(), w.contiguous()
-    dx, dw = torch.empty_like(x), torch.empty_like(w)
+    dx, dw = torch.empty_like(x), torch.empty_like(w, dtype=sum_dtype)
     rows, H = _rows(x), x.shape[-1]
     scratch = norm_bwd_scratch(rows, H, x.device)
     _check(load().jpb_norm_bwd(0, _dt(x), dy.data_ptr(), x.data_ptr(), w.data_ptr(), None, rstd.data_ptr(), dx.data_ptr(),
-                               dw.data_ptr(), None, scratch.data_ptr(), rows, H, _stream()), "rmsnorm_bwd", 2)
+                               dw.data_ptr(), None, scratch.data_ptr(), rows, H, _wide(sum_dtype, w), _stream()), "rmsnorm_bwd", 2)
     return dx, dw
 
 
-def _norm_bwd_add(layer, dy, x, w, mean, rstd, add):
+def _norm_bwd_add(layer, dy, x, w, mean, rstd, add, sum_dtype):
     dy, x, w, add = dy.contiguous(), x.contiguous(), w.contiguous(), add.contiguous()
     lib = load()
-    lib.jpb_norm_bwd_add.argtypes = [_c_int, _c_int] + [_c_p] * 9 + [_c_int, _c_int, _c_p, _c_p]
-    dx, dw = torch.empty_like(x), torch.empty_like(w)
-    db = torch.empty_like(w) if layer else None
+    lib.jpb_norm_bwd_add.argtypes = [_c_int, _c_int] + [_c_p] * 9 + [_c_int, _c_int, _c_p, _c_int, _c_p]
+    dx, dw = torch.empty_like(x), torch.empty_like(w, dtype=sum_dtype)
+    db = torch.empty_like(dw) if layer else None
     rows, H = _rows(x), x.shape[-1]
     scratch = norm_bwd_scratch(rows, H, x.device)
     _check(lib.jpb_norm_bwd_add(layer, _dt(x), dy.data_ptr(), x.data_ptr(), w.data_ptr(), _p(mean), rstd.data_ptr(),
-                                dx.data_ptr(), dw.data_ptr(), _p(db), scratch.data_ptr(), rows, H, add.data_ptr(), _stream()),
-           "norm_bwd_add", 2)
+                                dx.data_ptr(), dw.data_ptr(), _p(db), scratch.data_ptr(), rows, H, add.data_ptr(), _wide(sum_dtype, w),
+                                _stream()), "norm_bwd_add", 2)
     return (dx, dw, db) if layer else (dx, dw)
 
 
-def rmsnorm_bwd_add(dy, x, w, rstd, add):
-    return _norm_bwd_add(0, dy, x, w, None, rstd, add)
+def rmsnorm_bwd_add(dy, x, w, rstd, add, sum_dtype=None):
+    return _norm_bwd_add(0, dy, x, w, None, rstd, add, sum_dtype)
 
 
-def layernorm_bwd_add(dy, x, w, mean, rstd, add):
-    return _norm_bwd_add(1, dy, x, w, mean, rstd, add)
+def layernorm_bwd_add(dy, x, w, mean, rstd, add, sum_dtype=None):
+    return _norm_bwd_add(1, dy, x, w, mean, rstd, add, sum_dtype)
 
 
 def layernorm(x, w, b, eps):
@@ -361,23 +370,25 @@ def layernorm(x, w, b, eps):
     return y, mean, rstd
 
 
-def layernorm_bwd(dy, x, w, mean, rstd):
+def layernorm_bwd(dy, x, w, mean, rstd, sum_dtype=None):
     dy, x, w = dy.contiguous(), x.contiguous(), w.contiguous()
-    dx, dw, db = torch.empty_like(x), torch.empty_like(w), torch.empty_like(w)
+    dx, dw = torch.empty_like(x), torch.empty_like(w, dtype=sum_dtype)
+    db = torch.empty_like(dw)
     rows, H = _rows(x), x.shape[-1]
     scratch = norm_bwd_scratch(rows, H, x.device)
     _check(load().jpb_norm_bwd(1, _dt(x), dy.data_ptr(), x.data_ptr(), w.data_ptr(), mean.data_ptr(), rstd.data_ptr(),
-                               dx.data_ptr(), dw.data_ptr(), db.data_ptr(), scratch.data_ptr(), rows, H, _stream()),
-           "layernorm_bwd", 2)
+                               dx.data_ptr(), dw.data_ptr(), db.data_ptr(), scratch.data_ptr(), rows, H, _wide(sum_dtype, w),
+                               _stream()), "layernorm_bwd", 2)
     return dx, dw, db
 
 
-def colsum(dy):
+def colsum(dy, sum_dtype=None):
     dy = dy.contiguous()
     rows, cols = _rows(dy), dy.shape[-1]
-    out = torch.empty(cols, dtype=dy.dtype, device=dy.device)
+    out = torch.empty(cols, dtype=sum_dtype or dy.dtype, device=dy.device)
     scratch = torch.empty(load().jpb_colsum_scratch_elems(rows, cols), dtype=torch.float32, device=dy.device)
-    _check(load().jpb_colsum(_dt(dy), dy.data_ptr(), out.data_ptr(), scratch.data_ptr(), rows, cols, _stream()), "colsum", 2)
+    _check(load().jpb_colsum(_dt(dy), dy.data_ptr(), out.data_ptr(), scratch.data_ptr(), rows, cols, _wide(sum_dtype, dy), _stream()),
+           "colsum", 2)
     return out
 
 

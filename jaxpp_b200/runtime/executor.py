@@ -79,9 +79,29 @@ class RankState:
         self.record_events = record_events and device.type == "cuda"
         self.events: list[tuple[str, Any, Any]] = []
         self.pending_events: dict[int, Any] = {}   # value id -> CUDA event of the side-stream work that produces it
+        # accumulations that nothing has read yet (accumulator, contribution): bias and norm gradients come in runs of
+        # dozens of small additions, which leave as one multi-tensor addition per dtype
+        self.adds: list[tuple[torch.Tensor, torch.Tensor]] = []
+
+    def flush(self):
+        """Carry out the additions put off by :meth:`accum`; called before anything else of this rank runs or is read."""
+        adds, self.adds = self.adds, []
+        if len(adds) < 2:
+            for acc, val in adds:
+                acc.add_(val)
+            return
+        groups: dict = {}
+        for acc, val in adds:
+            groups.setdefault((acc.dtype, val.dtype), ([], []))
+            groups[acc.dtype, val.dtype][0].append(acc)
+            groups[acc.dtype, val.dtype][1].append(val)
+        for accs, vals in groups.values():
+            torch._foreach_add_(accs, vals)
 
     # -- individual instructions --------------------------------------------------------------
     def run_task(self, ins: RunTask):
+        if self.adds:
+            self.flush()
         env = self.env
         args = []
         for v, donate in zip(ins.ins, ins.donate):
@@ -154,6 +174,8 @@ class RankState:
         return run
 
     def slice(self, ins: Slice):
+        if self.adds:
+            self.flush()
         self.env[ins.out] = self.env[ins.src].select(ins.axis, ins.index)
 
     def loop_index(self, ins: LoopIndex):
@@ -167,6 +189,8 @@ class RankState:
         env = self.env
         val = env[ins.val]
         acc = env.get(ins.acc)
+        if self.adds and (ins.kind != 0 or any(acc is a or val is a or acc is v for a, v in self.adds)):
+            self.flush()
         if ins.kind == 1:  # concat: write slot
             if acc is None:
                 shape = list(val.shape)
@@ -180,7 +204,11 @@ class RankState:
         elif acc is val:
             pass  # the task already added this microbatch's contribution into the accumulator (a sink)
         elif ins.kind == 0:
-            acc.add_(val)
+            # a large addition gains nothing from waiting, and its operands would stay alive meanwhile
+            if val.numel() <= 1 << 16 and val.shape == acc.shape and val.device == acc.device:
+                self.adds.append((acc, val))
+            else:
+                acc.add_(val)
         else:
             torch.maximum(acc, val, out=acc)
 
@@ -247,6 +275,7 @@ def run_single_controller(prog: Program, inputs: Sequence[torch.Tensor | None], 
         elif isinstance(ins, Accum):
             st.accum(ins)
         elif isinstance(ins, Transfer):
+            st.flush()
             dst = states[ins.dst]
             for v in ins.vids:
                 t = st.env[v]
@@ -257,6 +286,7 @@ def run_single_controller(prog: Program, inputs: Sequence[torch.Tensor | None], 
             st.delete(ins)
         elif isinstance(ins, (AllReduce, AllGather)):
             # a rank's contribution is read when *its* instruction is reached (it may be deleted right after)
+            st.flush()
             group = pending_collectives[ins.cid]
             if isinstance(ins, AllReduce):
                 info = prog.values[ins.out]
@@ -270,6 +300,8 @@ def run_single_controller(prog: Program, inputs: Sequence[torch.Tensor | None], 
             raise NotImplementedError(type(ins))
     if track:
         LIVE_REPORT.append(peak)
+    for st in states:
+        st.flush()
     outs = []
     for o in prog.outputs:
         if o[0] == "c":
@@ -337,6 +369,7 @@ def run_multi_controller(prog: Program, rank: int, inputs: Sequence[torch.Tensor
             comm.before_use(st, (ins.val,))
             st.accum(ins)
         elif isinstance(ins, Transfer):
+            st.flush()
             if ins.rank == rank:
                 comm.send(st, ins, prog)
             else:
@@ -346,15 +379,18 @@ def run_multi_controller(prog: Program, rank: int, inputs: Sequence[torch.Tensor
         elif isinstance(ins, Delete):
             st.delete(ins)
         elif isinstance(ins, AllReduce):
+            st.flush()
             comm.before_use(st, ins.local)
             info = prog.values[ins.out]
             buf = _local_sum(st, ins, info.shape, info.dtype)
             st.env[ins.out] = comm.all_reduce(buf, ins.ranks)
         elif isinstance(ins, AllGather):
+            st.flush()
             comm.before_use(st, ins.local.values())
             st.env[ins.out] = comm.all_gather(st, ins, prog)
         else:  # pragma: no cover
             raise NotImplementedError(type(ins))
+    st.flush()
     comm.end_step(st)
     if track:
         peak["rank"] = rank
