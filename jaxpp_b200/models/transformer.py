@@ -444,6 +444,9 @@ class _Recompute(torch.autograd.Function):
             out = fn(*args)
         ctx.save_for_backward(*[a for a in args if isinstance(a, torch.Tensor)])
         ctx.is_tensor = [isinstance(a, torch.Tensor) for a in args]
+        # parameters whose gradients are wanted in another type than their own (fp32 gradients of bf16 weights): the re-run
+        # must ask for that type too, or every weight gradient is rounded to bf16 by one pass and widened by another
+        ctx.grad_dtypes = [a.grad_dtype if isinstance(a, torch.Tensor) and a.is_leaf and a.requires_grad else None for a in args]
         ctx.others = [a for a in args if not isinstance(a, torch.Tensor)]
         return out
 
@@ -451,10 +454,12 @@ class _Recompute(torch.autograd.Function):
     def backward(ctx, *gs):
         saved, others = list(ctx.saved_tensors), list(ctx.others)
         args = []
-        for is_t in ctx.is_tensor:
+        for is_t, grad_dtype in zip(ctx.is_tensor, ctx.grad_dtypes):
             if is_t:
                 a = saved.pop(0)
                 args.append(a.detach().requires_grad_(a.is_floating_point()))
+                if grad_dtype is not None and grad_dtype != a.dtype:
+                    args[-1].grad_dtype = grad_dtype
             else:
                 args.append(others.pop(0))
         with torch.enable_grad():
