@@ -585,6 +585,66 @@ __global__ void embedding_bwd_kernel(const T* __restrict__ dy, const int64_t* __
   }
 }
 
+// The same gradient for a bf16 table, without an fp32 staging table of its size: the tokens of every id are collected in a
+// list (three passes over the ids), and the CTAs of an id's first token add up its rows in fp32 registers and write, or add
+// to, the table's row once.  Bound by the rows of dy and the touched rows of the table (32000 x 8192, 4096 tokens: 67 MB
+// each way; clearing, scattering into and casting an fp32 table moved 2.7 GB, 1.07 ms).
+struct EmbLists {
+  int* count;    // [vocab] tokens per id, zero on entry; count[vocab]: tokens placed so far
+  int* base;     // [vocab] start of an id's list (of ids that occur)
+  int* rank;     // [n_tok] position of a token in its id's list, -1: id out of range
+  int* list;     // [n_tok]
+};
+__global__ void emb_count_kernel(const int64_t* __restrict__ ids, EmbLists l, int n_tok, int vocab) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= n_tok) return;
+  const int64_t id = ids[t];
+  l.rank[t] = id < 0 || id >= vocab ? -1 : atomicAdd(&l.count[id], 1);
+}
+__global__ void emb_base_kernel(const int64_t* __restrict__ ids, EmbLists l, int n_tok, int vocab) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= n_tok || l.rank[t] != 0) return;
+  l.base[ids[t]] = atomicAdd(&l.count[vocab], l.count[ids[t]]);
+}
+__global__ void emb_list_kernel(const int64_t* __restrict__ ids, EmbLists l, int n_tok) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= n_tok || l.rank[t] < 0) return;
+  l.list[l.base[ids[t]] + l.rank[t]] = t;
+}
+constexpr int EMB_THREADS = 128;
+__global__ void __launch_bounds__(EMB_THREADS) emb_sum_kernel(const __nv_bfloat16* __restrict__ dy, const int64_t* __restrict__ ids, EmbLists l,
+                                                              __nv_bfloat16* __restrict__ table, int d, int accumulate) {
+  constexpr int VN = Vec<__nv_bfloat16>::N;
+  const int t = blockIdx.x;
+  if (l.rank[t] != 0) return;
+  const int64_t id = ids[t];
+  const int n = l.count[id];
+  const int* list = l.list + l.base[id];
+  const int c = (blockIdx.y * EMB_THREADS + threadIdx.x) * VN;
+  if (c >= d) return;
+  float acc[VN];
+#pragma unroll
+  for (int j = 0; j < VN; ++j) acc[j] = 0.f;
+#pragma unroll 4
+  for (int i = 0; i < n; ++i) {
+    Vec<__nv_bfloat16> v; v.load(dy + size_t(list[i]) * d + c);
+    float f[VN]; v.to_float(f);
+#pragma unroll
+    for (int j = 0; j < VN; ++j) acc[j] += f[j];
+  }
+  __nv_bfloat16* row = table + size_t(id) * d + c;
+  Vec<__nv_bfloat16> o; o.from_float(acc);
+  if (accumulate) {   // the sum is rounded before it is added, as a gradient tensor of its own would be
+    Vec<__nv_bfloat16> old; old.load(row);
+    float a[VN], b[VN];
+    old.to_float(a); o.to_float(b);
+#pragma unroll
+    for (int j = 0; j < VN; ++j) a[j] += b[j];
+    o.from_float(a);
+  }
+  o.store(row);
+}
+
 template <typename T>
 __global__ void cast_from_f32_kernel(const float* __restrict__ in, T* __restrict__ out, size_t n) {
   for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += size_t(gridDim.x) * blockDim.x)
@@ -1012,6 +1072,29 @@ JPB_API int jpb_embedding_bwd_acc(int dt, const void* dy, const long long* ids, 
     embedding_bwd_kernel<T><<<ew_grid(work, 256), 256, 0, STREAM>>>((const T*)dy, (const int64_t*)ids, acc, n_tok, d, vocab);
     return LAST_ERR;
   });
+}
+
+// Gradient of a bf16 table [vocab, d] from bf16 rows, cleared first or added to.  `scratch`: 2 * vocab + 1 + 2 * n_tok ints.
+JPB_API int jpb_embedding_bwd_bf16(const void* dy, const long long* ids, void* table, int* scratch, int n_tok, int d, int vocab,
+                                   int accumulate, void* stream) {
+  if (d % Vec<__nv_bfloat16>::N || (reinterpret_cast<uintptr_t>(table) & 15)) return -int(JPB_ERR_BAD_ARGUMENT);
+  if (!accumulate) cudaMemsetAsync(table, 0, size_t(vocab) * d * sizeof(__nv_bfloat16), STREAM);
+  if (n_tok <= 0) return LAST_ERR;
+  EmbLists l;
+  l.count = scratch;
+  l.base = scratch + vocab + 1;
+  l.rank = l.base + vocab;
+  l.list = l.rank + n_tok;
+  cudaMemsetAsync(l.count, 0, size_t(vocab + 1) * sizeof(int), STREAM);
+  const int64_t* id = reinterpret_cast<const int64_t*>(ids);
+  const int blocks = (n_tok + 255) / 256;
+  emb_count_kernel<<<blocks, 256, 0, STREAM>>>(id, l, n_tok, vocab);
+  emb_base_kernel<<<blocks, 256, 0, STREAM>>>(id, l, n_tok, vocab);
+  emb_list_kernel<<<blocks, 256, 0, STREAM>>>(id, l, n_tok);
+  const int per = EMB_THREADS * Vec<__nv_bfloat16>::N;
+  emb_sum_kernel<<<dim3(n_tok, (d + per - 1) / per), EMB_THREADS, 0, STREAM>>>(static_cast<const __nv_bfloat16*>(dy), id, l,
+                                                                               static_cast<__nv_bfloat16*>(table), d, accumulate);
+  return LAST_ERR;
 }
 
 JPB_API int jpb_ce_fwd(int dt, const void* logits, const long long* labels, float* loss, float* lse, int rows, int V,

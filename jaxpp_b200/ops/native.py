@@ -483,11 +483,25 @@ def embedding(ids, table):
 
 def embedding_bwd(dy, ids, vocab, out_dtype=None, out: Optional[torch.Tensor] = None, accumulate: bool = False):
     """Gradient of the embedding table: rows of ``dy`` summed by token id.  ``out_dtype`` float32 returns the fp32 sum
-    itself (no cast pass); with ``out`` (fp32 [vocab, d]) the rows are added into it (``accumulate``) or it is
-    cleared first."""
+    itself (no cast pass); with ``out`` (fp32, or bf16 like ``dy``, [vocab, d]) the rows are added into it (``accumulate``)
+    or it is cleared first."""
     dy, ids = dy.contiguous(), ids.contiguous()
     d = dy.shape[-1]
     want = out_dtype or dy.dtype
+    # Without an fp32 table in between from 8 M elements on: three more launches (8 us) against 8 bytes per element less
+    # memory traffic (1.2 us per million elements).  A bf16 accumulator only has this path.
+    if dy.dtype == torch.bfloat16 and d % 8 == 0 and (
+            out.dtype == torch.bfloat16 if out is not None else want == torch.bfloat16 and vocab * d >= 8 << 20):
+        lib = load()
+        lib.jpb_embedding_bwd_bf16.argtypes = [_c_p, _c_p, _c_p, _c_p, _c_int, _c_int, _c_int, _c_int, _c_p]
+        table = out if out is not None else torch.empty(vocab, d, dtype=torch.bfloat16, device=dy.device)
+        if not table.is_contiguous():
+            raise NativeError("embedding_bwd accumulates into a contiguous table")
+        n = ids.numel()
+        scratch = torch.empty(2 * vocab + 1 + 2 * n, dtype=torch.int32, device=dy.device)
+        _check(lib.jpb_embedding_bwd_bf16(dy.data_ptr(), ids.data_ptr(), table.data_ptr(), scratch.data_ptr(), n, d, vocab,
+                                          int(accumulate), _stream()), "embedding_bwd", 4)
+        return table
     if out is not None or want == torch.float32:
         lib = load()
         lib.jpb_embedding_bwd_acc.argtypes = [_c_int, _c_p, _c_p, _c_p, _c_ll, _c_int, _c_int, _c_int, _c_p]

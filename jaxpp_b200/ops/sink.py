@@ -49,7 +49,9 @@ def accumulate(op, acc: torch.Tensor, *args, **kwargs) -> torch.Tensor:
             return acc
     elif op is torch.ops.b200.embedding_bwd.default:
         dy, ids, vocab = args[0], args[1], args[2]
-        if (ops._use_native(dy) and acc.dtype == torch.float32 and acc.is_contiguous() and acc.dim() == 2
+        wide = acc.dtype == torch.float32
+        narrow = acc.dtype == dy.dtype == torch.bfloat16 and acc.shape[-1] % 8 == 0 and acc.data_ptr() % 16 == 0
+        if (ops._use_native(dy) and (wide or narrow) and acc.is_contiguous() and acc.dim() == 2
                 and acc.shape[0] == vocab and acc.shape[1] == dy.shape[-1]):
             ops._native().embedding_bwd(dy, ids, vocab, out=acc, accumulate=True)   # scatter-add into the accumulator
             return acc

@@ -374,6 +374,27 @@ def test_adamw_with_clip_coefficient(native, n, offset, gdt):
         assert torch.equal(got[3], got[0].to(torch.bfloat16))
 
 
+@pytest.mark.parametrize("vocab,d,n", [(8200, 1032, 700), (9000, 1024, 1), (70000, 128, 3000)])
+def test_embedding_gradient_of_a_bf16_table(native, vocab, d, n):
+    """Lists of tokens per id: ids that occur once, never and hundreds of times, more than one CTA per row, out of range;
+    a table of its own and an accumulator.  One fp32 chain per element, rounded to bf16 (2^-9)."""
+    g = torch.Generator().manual_seed(3)
+    ids = torch.randint(0, vocab, (n,), generator=g)
+    ids[: n // 2] = 17
+    if n > 100:
+        ids[5], ids[6] = -1, vocab
+    ids, dy = ids.cuda(), rnd(n, d, seed=6)
+    ok = (ids >= 0) & (ids < vocab)
+    want = torch.zeros(vocab, d, dtype=torch.float64, device="cuda").index_add_(0, ids[ok], dy[ok].double())
+    slack = n * 2.0 ** -23 * torch.zeros_like(want).index_add_(0, ids[ok], dy[ok].double().abs())
+    got = native.embedding_bwd(dy, ids, vocab)
+    assert got.dtype == torch.bfloat16 and ((got.double() - want).abs() <= slack + 2.0 ** -8 * want.abs()).all()
+    acc = rnd(vocab, d, seed=7)
+    expected = acc.float() + got.float()         # what adding the gradient as a tensor gives, but for the order of the sums
+    native.embedding_bwd(dy, ids, vocab, out=acc, accumulate=True)
+    assert ((acc.float() - expected).abs() <= 2.0 ** -7 * (expected.abs() + got.float().abs()) + 1e-6).all()
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_dropout_matches_counter_based_reference(native, dtype):
     from jaxpp_b200.ops import core as ops
