@@ -8,6 +8,7 @@ from __future__ import annotations
 
 import ctypes
 import os
+import threading
 from typing import Optional
 
 import torch
@@ -558,6 +559,16 @@ def sum_squares(tensors):
     return out
 
 
+# addresses that in-place ops of a step being recorded write to (see runtime/replay.py); None outside of a recording
+_recording = threading.local()
+
+
+def log_in_place(*tensors) -> None:
+    seen = getattr(_recording, "written", None)
+    if seen is not None:
+        seen.update(t.data_ptr() for t in tensors if t is not None)
+
+
 def adamw(master, grad, m, v, step, lr, beta1, beta2, eps, weight_decay, grad_scale, out_dtype, lp_old=None,
           inplace=False, clip=None):
     grad = grad.contiguous()
@@ -568,6 +579,7 @@ def adamw(master, grad, m, v, step, lr, beta1, beta2, eps, weight_decay, grad_sc
             raise NativeError("in-place adamw needs contiguous state tensors")
         p2, m2, v2 = master, m, v
         reuse = lp_old is not None and lp_old.dtype == out_dtype and lp_old.is_contiguous()
+        log_in_place(master, m, v, lp_old if reuse else None)
         lp = lp_old if reuse else torch.empty(master.shape, dtype=out_dtype, device=master.device)
     else:
         master, m, v = master.contiguous(), m.contiguous(), v.contiguous()

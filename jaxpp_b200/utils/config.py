@@ -169,6 +169,8 @@ overlap_collective_ctas = IntEnvVar("JAXPP_B200_OVERLAP_CTAS", 32)
 # input-gradient GEMMs (faster only when empty tiles come in runs that keep the CTAs' walk over the tiles in step:
 # 1.7x at 50 % fill, nothing at 80 % fill in one block per expert).
 moe_skip_empty_slots = IntEnvVar("JAXPP_B200_MOE_SKIP_EMPTY_SLOTS", 1)
+# Replay launch-bound single-process steps as CUDA graphs from their third call on (runtime/replay.py).
+step_graphs = BoolEnvVar("JAXPP_B200_STEP_GRAPHS", True)
 # Seconds a rank may go without a heartbeat before the watchdog reports it.
 heartbeat_timeout_s = IntEnvVar("JAXPP_B200_HEARTBEAT_TIMEOUT", 30)
 # Wrap every task in an NVTX range named like the task (fwd_3__5, …) for timeline profilers.
