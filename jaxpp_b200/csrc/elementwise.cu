@@ -881,14 +881,15 @@ JPB_API int jpb_norm_fwd(int layer, int dt, const void* x, const void* w, const 
   });
 }
 
-// CTAs of the norm backward: enough to keep about 1024 threads per SM (a row of 1600 bf16 is a CTA of 128 threads, and
-// two of those per SM left the memory system idle most of the time: 16384 rows took 121 us), but eight rows or more
-// each beyond two per SM, since every CTA leaves 2 H partial sums behind.
+// CTAs of the norm backward: as many as are resident at once (its 128 registers per thread leave room for 512 threads per
+// SM), since every CTA leaves 2 H partial sums behind and a second wave would be a ragged one.  A row of 1600 bf16 is a CTA
+// of 128 threads, and two of those per SM left the memory system idle: 16384 rows took 139 us, with four 85, with eight, half of them waiting, 101;
+// rows of 4096 (256 threads) take 42 us with two per SM and 50 with up to four.  Few rows: two per SM.
 static int norm_bwd_grid(int rows, int H, int vn) {
   const int threads = norm_threads(H, vn, NORM_BWD_VECS);
-  const int per_sm = threads >= 512 ? 2 : 1024 / threads < 8 ? 1024 / threads : 8;
-  int grid = sm_count() * 2;
-  if (rows / 8 > grid) grid = rows / 8 < sm_count() * per_sm ? rows / 8 : sm_count() * per_sm;
+  const int per_sm = threads > 128 ? 2 : 512 / threads < 8 ? 512 / threads : 8;
+  const int full = sm_count() * per_sm;
+  const int grid = rows >= 4 * full ? full : sm_count() * 2;
   return rows < grid ? rows : grid;
 }
 
