@@ -23,10 +23,10 @@ from ..compiler.program import Accum, Delete, Program, RunTask, SendDone, Slice
 from ..utils import config, logger, optimes
 from .. import fault
 
-# The copies cost 2 x bytes / HBM bandwidth per call (64 MB: about 20 us) and the op-by-op launches that they replace at
-# least 10 us per kernel; with larger inputs a step is bound by its kernels and the memory kept here would count.
-MAX_INPUT_BYTES = 64 << 20
-MAX_OUTPUT_BYTES = 128 << 20
+# The copies in and back cost 4 x bytes / HBM bandwidth per call (1 MB: 0.6 us) and the op-by-op launches that they replace
+# at least 10 us per op: 64 MB (40 us) are always worth it, and 1 MB per op beyond.  With more than MAX_BYTES a step is
+# bound by its kernels and the memory kept here would count.
+FREE_BYTES, BYTES_PER_OP, MAX_BYTES = 64 << 20, 1 << 20, 256 << 20
 MIN_OPS = 8
 MAX_POOL_BYTES = 512 << 20       # memory that one recording may keep for its intermediate values
 TOTAL_POOL_BYTES = 1 << 30       # and all recordings of the process together
@@ -77,7 +77,7 @@ def _program_ok(prog: Program) -> bool:
             return False
     in_bytes = sum(prog.values[vid].nbytes for vid, ranks in prog.inputs if ranks)
     out_bytes = sum(prog.values[o[1]].nbytes for o in prog.outputs if o[0] != "c")
-    return ops >= MIN_OPS and in_bytes <= MAX_INPUT_BYTES and out_bytes <= MAX_OUTPUT_BYTES
+    return ops >= MIN_OPS and max(in_bytes, out_bytes) <= min(MAX_BYTES, FREE_BYTES + ops * BYTES_PER_OP)
 
 
 def _plain(x, device: torch.device) -> bool:
