@@ -559,14 +559,15 @@ def sum_squares(tensors):
     return out
 
 
-# addresses that in-place ops of a step being recorded write to (see runtime/replay.py); None outside of a recording
+# storages that in-place ops of a step being recorded write to (see runtime/replay.py); None outside of a recording.  By
+# storage: an op may update a view that starts anywhere in an input.
 _recording = threading.local()
 
 
 def log_in_place(*tensors) -> None:
     seen = getattr(_recording, "written", None)
     if seen is not None:
-        seen.update(t.data_ptr() for t in tensors if t is not None)
+        seen.update(t.untyped_storage().data_ptr() for t in tensors if t is not None)
 
 
 def adamw(master, grad, m, v, step, lr, beta1, beta2, eps, weight_decay, grad_scale, out_dtype, lp_old=None,

@@ -89,6 +89,12 @@ def _same_memory(a: torch.Tensor, b: torch.Tensor) -> bool:
     return a.data_ptr() == b.data_ptr() and a.shape == b.shape and a.stride() == b.stride() and a.dtype == b.dtype
 
 
+def _overlap(tensors: Sequence) -> bool:
+    """Do any two of these contiguous tensors share memory?"""
+    spans = sorted((x.data_ptr(), x.nbytes) for x in tensors if x is not None and x.numel())
+    return any(a + n > b for (a, n), (b, _) in zip(spans, spans[1:]))
+
+
 def _copy_all(dst: list, src: list) -> None:
     """One multi-tensor copy per dtype."""
     groups: dict = {}
@@ -134,7 +140,9 @@ class _Recording:
         self.launches = native.LAUNCHES[0] - launches
         native.LAUNCHES[0] = launches
         self.pool_bytes = max(0, torch.cuda.memory_reserved(device) - before)
-        self.written = [k for k, s in enumerate(self.static) if s is not None and (s.data_ptr() in written or s._version != versions[k])]
+        # (every static tensor has a storage of its own)
+        self.written = [k for k, s in enumerate(self.static)
+                        if s is not None and (s.untyped_storage().data_ptr() in written or s._version != versions[k])]
         # every output: a constant, an input (passed through or updated in place), or the n-th result of the graph
         self.results: list = []
         self.outputs: list = []
@@ -228,8 +236,8 @@ class StepReplay:
                 rec = self._record(inputs, device, execute)
             if rec is None or rec.settings != _settings() or rec.device != device:
                 return None
-            if rec.written and len({x.data_ptr() for x in inputs if x is not None}) < sum(x is not None for x in inputs):
-                return None      # one buffer given twice and updated in place: the order of the updates matters
+            if rec.written and _overlap(inputs):
+                return None      # an update in place of one input is seen through another: the order of the updates matters
             return rec.run(inputs)
 
     def _record(self, inputs, device, execute) -> _Recording | None:

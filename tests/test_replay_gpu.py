@@ -8,6 +8,7 @@ from torch.utils import _pytree as pytree
 import jaxpp_b200 as jp
 from jaxpp_b200.models import lm_trainer as lt
 from jaxpp_b200.models import transformer as tf
+from jaxpp_b200.ops import core as ops
 from jaxpp_b200.utils import config
 
 pytestmark = pytest.mark.gpu
@@ -135,3 +136,37 @@ def test_calls_that_a_recording_does_not_cover_run_op_by_op():
     for _ in range(4):
         big(wide, square)
     assert _replay(big).recording is None
+
+
+def _update_slices(flat, other, m, v, g, step):
+    n = flat.shape[0] // 2
+    out = []
+    for lo, hi in ((8, n), (n, 2 * n)):      # parameters that live in one flat buffer of fp32 state
+        _, _, _, lp = ops.adamw(flat[lo:hi], g[lo:hi], m[lo:hi], v[lo:hi], step, 1e-2, 0.9, 0.95, 1e-8, 0.1, 1.0, torch.bfloat16, None, True)
+        out.append(lp * 2 + 1)
+    return jp.mark_stage_end((*out, flat, other + 1))
+
+
+@pytest.mark.parametrize("aliased", [False, True])
+def test_updates_in_place_of_views_reach_the_callers_buffers(aliased):
+    """The step updates slices at an offset of its inputs; with ``aliased`` another input overlaps the updated buffer."""
+    step, eager = (jp.mpmd_jit_by_yield(_update_slices, _mesh()) for _ in range(2))
+    n = 1024
+
+    def fresh():
+        gen = torch.Generator(device="cuda").manual_seed(4)
+        buf = torch.randn(4 * n, generator=gen, device="cuda")
+        m, g = torch.randn(2, 2 * n, generator=gen, device="cuda").unbind(0)
+        v = torch.rand(2 * n, generator=gen, device="cuda")
+        other = buf[n:3 * n] if aliased else buf[2 * n:4 * n]
+        return buf[:2 * n], other, m.clone(), v, g.clone(), torch.tensor(3, device="cuda")
+
+    a, b = fresh(), fresh()
+    for _ in range(6):
+        got = _tensors(step(*a))
+        with config.step_graphs.set(False):
+            want = _tensors(eager(*b))
+        for x, y in zip((*got, *a), (*want, *b)):
+            assert torch.equal(x, y)
+        assert got[2].data_ptr() == a[0].data_ptr()
+    assert _replay(step).recording is not None
