@@ -38,12 +38,17 @@ __device__ __forceinline__ float as_float(__nv_bfloat16 v) { return __bfloat162f
 // ---------------------------------------------------------------------------------------------------------
 // Router: softmax over the expert logits, top-k pick, weights renormalised over the picks, and the two
 // per-expert statistics of the load-balancing loss (sum of probabilities, number of picks) in one pass.
-// One thread per token, its probabilities in registers: EP is E rounded up to a power of two.
+// One thread per token, its probabilities in registers: EP is E rounded up to a power of two.  A CTA leaves the sums of
+// its tokens' probabilities in its own row of `part` (may be absent), so that the loss is a sum in a fixed order: the same
+// bits on every run.  The picks are counted in whole numbers, whose order does not matter.
 // ---------------------------------------------------------------------------------------------------------
+constexpr int ROUTER_THREADS = 64;
 template <typename T, int EP>
-__global__ void router_kernel(const T* __restrict__ logits, float* __restrict__ probs, long long* __restrict__ top_i,
-                              float* __restrict__ weights, float* __restrict__ prob_sum, float* __restrict__ hits, int n_tok,
-                              int E, int k, int* status) {
+__global__ void __launch_bounds__(ROUTER_THREADS)
+router_kernel(const T* __restrict__ logits, float* __restrict__ probs, long long* __restrict__ top_i, float* __restrict__ weights,
+              float* __restrict__ part, float* __restrict__ hits, int n_tok, int E, int k, int* status) {
+  __shared__ float sums[ROUTER_THREADS / 32][EP];
+  __shared__ int counts[ROUTER_THREADS / 32][EP];
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   const bool in = t < n_tok;
   float p[EP];
@@ -94,27 +99,58 @@ __global__ void router_kernel(const T* __restrict__ logits, float* __restrict__ 
     top_i[size_t(t) * k + j] = idx[j];
     weights[size_t(t) * k + j] = val[j] * pinv;
   }
-  const int lane = threadIdx.x & 31;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (!in) taken = 0ull;
 #pragma unroll
   for (int e = 0; e < EP; ++e) {
     if (e >= E) break;
     const float s = warp_sum(p[e]);
     const int c = __popc(__ballot_sync(0xffffffffu, (taken >> e) & 1ull));
-    if (lane == 0) {
-      atomicAdd(prob_sum + e, s);
-      if (c) atomicAdd(hits + e, float(c));
-    }
+    if (lane == 0) { sums[warp][e] = s; counts[warp][e] = c; }
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < E; e += ROUTER_THREADS) {
+    float s = 0.f;
+    int c = 0;
+#pragma unroll
+    for (int w = 0; w < ROUTER_THREADS / 32; ++w) { s += sums[w][e]; c += counts[w][e]; }
+    if (part) part[size_t(blockIdx.x) * E + e] = s;
+    if (c) atomicAdd(hits + e, float(c));
   }
 }
 
-// aux = scale * sum_e hits[e] * prob_sum[e]
-__global__ void router_aux_kernel(const float* __restrict__ prob_sum, const float* __restrict__ hits, float* __restrict__ aux, int E,
-                                  float scale) {
-  float s = 0.f;
-  for (int e = threadIdx.x; e < E; e += 32) s += hits[e] * prob_sum[e];
-  s = warp_sum(s);
-  if (threadIdx.x == 0) *aux = s * scale;
+// aux = scale * sum_e hits[e] * (sum of column e of part).  AUX_THREADS / EP threads share a column, EP being E rounded up
+// to a power of two; their sums, and then the experts', meet in trees.  Bound by the latency of a thread's chain of loads,
+// of which four are in flight: 8192 tokens of 8 experts are 128 rows, one load a thread.
+constexpr int AUX_THREADS = 1024;
+__global__ void __launch_bounds__(AUX_THREADS) router_aux_kernel(const float* __restrict__ part, const float* __restrict__ hits,
+                                                                 float* __restrict__ aux, int rows, int E, int EP, float scale) {
+  __shared__ float red[AUX_THREADS];
+  const int e = threadIdx.x & (EP - 1), slice = threadIdx.x / EP, slices = AUX_THREADS / EP;
+  float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
+  if (e < E) {
+    int r = slice;
+    for (; r + 3 * slices < rows; r += 4 * slices) {
+      a0 += part[size_t(r) * E + e];
+      a1 += part[size_t(r + slices) * E + e];
+      a2 += part[size_t(r + 2 * slices) * E + e];
+      a3 += part[size_t(r + 3 * slices) * E + e];
+    }
+    for (; r < rows; r += slices) a0 += part[size_t(r) * E + e];
+  }
+  red[threadIdx.x] = (a0 + a1) + (a2 + a3);
+  __syncthreads();
+  for (int n = AUX_THREADS / 2; n >= EP; n >>= 1) {
+    if (threadIdx.x < n) red[threadIdx.x] += red[threadIdx.x + n];
+    __syncthreads();
+  }
+  if (threadIdx.x < EP) red[threadIdx.x] *= e < E ? hits[e] : 0.f;
+  __syncthreads();
+  for (int n = EP / 2; n >= 1; n >>= 1) {
+    if (threadIdx.x < n) red[threadIdx.x] += red[threadIdx.x + n];
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) *aux = red[0] * scale;
 }
 
 // Gradient of the logits from those of the weights (w_j = p_{i_j} / S, S the sum of the picked probabilities), of the
@@ -301,36 +337,41 @@ static bool aligned(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15
 
 }  // namespace jpb
 
+// fp32 elements of scratch that the loss of jpb_router needs: one row of E sums per CTA.
+JPB_API long long jpb_router_scratch_elems(int n_tok, int E) {
+  return (long long)((n_tok + jpb::ROUTER_THREADS - 1) / jpb::ROUTER_THREADS) * E;
+}
+
 // logits [n_tok, E] (fp32 dtype 0 or bf16 dtype 1) -> probs [n_tok, E] fp32, top_i [n_tok, k] int64, weights [n_tok, k]
-// fp32, prob_sum [E] and hits [E] fp32 (adjacent, both zeroed here), aux (one fp32, may be absent) =
-// aux_scale * sum_e hits[e] * prob_sum[e].  E <= 64, k <= 8.  A token whose probabilities are not
+// fp32, hits [E] fp32 (zeroed here), aux (one fp32, may be absent) = aux_scale * sum_e hits[e] * sum_t probs[t][e], which
+// needs `part`, jpb_router_scratch_elems() of scratch.  E <= 64, k <= 8.  A token whose probabilities are not
 // finite gets the lowest-numbered experts (indices stay in range) and the status word is set to JPB_ERR_BAD_ARGUMENT.
-JPB_API int jpb_router(int dtype, const void* logits, float* probs, long long* top_i, float* weights, float* prob_sum,
+JPB_API int jpb_router(int dtype, const void* logits, float* probs, long long* top_i, float* weights, float* part,
                        float* hits, float* aux, float aux_scale, int n_tok, int E, int k, void* stream) {
   using namespace jpb;
-  if (E < 1 || E > MOE_MAX_E || k < 1 || k > MOE_MAX_K || k > E) return -JPB_ERR_BAD_ARGUMENT;
+  if (E < 1 || E > MOE_MAX_E || k < 1 || k > MOE_MAX_K || k > E || (aux && n_tok > 0 && !part)) return -JPB_ERR_BAD_ARGUMENT;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (hits == prob_sum + E) {
-    cudaMemsetAsync(prob_sum, 0, sizeof(float) * 2 * E, s);
-  } else {
-    cudaMemsetAsync(prob_sum, 0, sizeof(float) * E, s);
-    cudaMemsetAsync(hits, 0, sizeof(float) * E, s);
-  }
-  if (n_tok > 0) {
-    const int threads = 64, blocks = (n_tok + threads - 1) / threads;
+  cudaMemsetAsync(hits, 0, sizeof(float) * E, s);
+  const int threads = ROUTER_THREADS, blocks = n_tok > 0 ? (n_tok + threads - 1) / threads : 0;
+  if (blocks) {
+    float* sums = aux ? part : nullptr;
     int* status = jpb_status_device_ptr();
     const int rc = by_dtype(dtype, [&](auto tag) {
       using T = decltype(tag);
       const T* lg = static_cast<const T*>(logits);
-      if (E <= 8) router_kernel<T, 8><<<blocks, threads, 0, s>>>(lg, probs, top_i, weights, prob_sum, hits, n_tok, E, k, status);
-      else if (E <= 16) router_kernel<T, 16><<<blocks, threads, 0, s>>>(lg, probs, top_i, weights, prob_sum, hits, n_tok, E, k, status);
-      else if (E <= 32) router_kernel<T, 32><<<blocks, threads, 0, s>>>(lg, probs, top_i, weights, prob_sum, hits, n_tok, E, k, status);
-      else router_kernel<T, 64><<<blocks, threads, 0, s>>>(lg, probs, top_i, weights, prob_sum, hits, n_tok, E, k, status);
+      if (E <= 8) router_kernel<T, 8><<<blocks, threads, 0, s>>>(lg, probs, top_i, weights, sums, hits, n_tok, E, k, status);
+      else if (E <= 16) router_kernel<T, 16><<<blocks, threads, 0, s>>>(lg, probs, top_i, weights, sums, hits, n_tok, E, k, status);
+      else if (E <= 32) router_kernel<T, 32><<<blocks, threads, 0, s>>>(lg, probs, top_i, weights, sums, hits, n_tok, E, k, status);
+      else router_kernel<T, 64><<<blocks, threads, 0, s>>>(lg, probs, top_i, weights, sums, hits, n_tok, E, k, status);
       return 0;
     });
     if (rc) return rc;
   }
-  if (aux) router_aux_kernel<<<1, 32, 0, s>>>(prob_sum, hits, aux, E, aux_scale);
+  if (aux) {
+    int ep = 1;
+    while (ep < E) ep *= 2;
+    router_aux_kernel<<<1, AUX_THREADS, 0, s>>>(part, hits, aux, blocks, E, ep, aux_scale);
+  }
   return int(cudaGetLastError());
 }
 

@@ -204,6 +204,8 @@ def _native():
 
         p, i, f = ctypes.c_void_p, ctypes.c_int, ctypes.c_float
         lib.jpb_router.argtypes = [i, p, p, p, p, p, p, p, f, i, i, i, p]
+        lib.jpb_router_scratch_elems.argtypes = [i, i]
+        lib.jpb_router_scratch_elems.restype = ctypes.c_longlong
         lib.jpb_router_bwd.argtypes = [i, p, p, p, p, p, p, p, i, i, i, f, p]
         lib.jpb_moe_slots.argtypes = [p, p, p, p, i, i, i, p]
         lib.jpb_moe_dispatch_rows.argtypes = [i, p, p, p, i, i, i, p]
@@ -226,12 +228,13 @@ def _router_native(logits: Tensor, top_k: int, want_aux: bool):
     probs = torch.empty(T, E, dtype=torch.float32, device=dev)
     top_i = torch.empty(T, top_k, dtype=torch.int64, device=dev)
     weights = torch.empty(T, top_k, dtype=torch.float32, device=dev)
-    stats = torch.empty(2, E, dtype=torch.float32, device=dev)
+    hits = torch.empty(E, dtype=torch.float32, device=dev)
     aux = torch.empty((), dtype=torch.float32, device=dev) if want_aux else None
+    part = torch.empty(lib.jpb_router_scratch_elems(T, E), dtype=torch.float32, device=dev) if want_aux else None
     native._check(lib.jpb_router(native._dt(lg), lg.data_ptr(), probs.data_ptr(), top_i.data_ptr(), weights.data_ptr(),
-                                 stats.data_ptr(), stats.data_ptr() + 4 * E, native._p(aux), _aux_scale(T, E, top_k), T, E, top_k,
+                                 native._p(part), hits.data_ptr(), native._p(aux), _aux_scale(T, E, top_k), T, E, top_k,
                                  native._stream()), "jpb_router", 2 if want_aux else 1)
-    return top_i, weights, probs, stats[1], aux
+    return top_i, weights, probs, hits, aux
 
 
 _lib.define("router(Tensor logits, int top_k) -> (Tensor, Tensor, Tensor, Tensor)")

@@ -316,6 +316,21 @@ def test_route_tokens_kernel_matches_the_composition(native, T, E, k, dtype):
     assert (got.double() - want).norm() <= bound * want.norm()
 
 
+@pytest.mark.parametrize("T,E,k", [(1, 3, 1), (8192, 8, 2), (12000, 16, 2), (40000, 64, 8)])
+def test_load_balancing_loss_repeats_and_is_summed_in_trees(native, T, E, k):
+    """The same bits on every run, and no long chain of additions: a CTA's 64 tokens in 6 steps, a thread's share of the CTAs'
+    rows (2048 / E of them at a time, at most 4 x ceil(rows / (4 * 1024 / E')) with E' = E rounded up), 2 + 10 steps between
+    threads, 3 roundings of the products; every term is positive, so each step adds at most 2^-24 of the result."""
+    logits = rnd(T, E, seed=93)
+    run = lambda: torch.ops.b200moe.route_tokens(logits, k)
+    _, _, probs, hits, aux = run()
+    for _ in range(30):
+        assert torch.equal(run()[4], aux)
+    want = E / (T * k * T) * (hits.double() * probs.double().sum(0)).sum()
+    steps = 6 + -(-(-(-T // 64)) // (1024 // (1 << (E - 1).bit_length()))) + 2 + 10 + 3
+    assert abs(aux.double() - want) <= steps * 2.0 ** -24 * want
+
+
 @pytest.mark.parametrize("layer", [False, True])
 @pytest.mark.parametrize("rows,H", [(2400, 1600), (9500, 256), (4737, 4096), (300, 8192)])
 def test_norm_backward_over_many_rows(native, layer, rows, H):
