@@ -168,6 +168,11 @@ class _Recording:
                 self.results.append(t)
             self.outputs.append(("out", rank, n))
 
+    def covers(self, inputs: Sequence) -> bool:
+        """A compiled step runs on whatever tensors it is called with; the recording is one of these shapes and dtypes."""
+        return all(x is s or (x is not None and s is not None and x.dtype == s.dtype and x.shape == s.shape)
+                   for x, s in zip(inputs, self.static))
+
     def run(self, inputs: Sequence) -> list:
         from ..ops import native
 
@@ -234,7 +239,7 @@ class StepReplay:
                 if self.calls <= EAGER_CALLS:
                     return None
                 rec = self._record(inputs, device, execute)
-            if rec is None or rec.settings != _settings() or rec.device != device:
+            if rec is None or rec.settings != _settings() or rec.device != device or not rec.covers(inputs):
                 return None
             if rec.written and _overlap(inputs):
                 return None      # an update in place of one input is seen through another: the order of the updates matters

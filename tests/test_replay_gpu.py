@@ -170,3 +170,20 @@ def test_updates_in_place_of_views_reach_the_callers_buffers(aliased):
             assert torch.equal(x, y)
         assert got[2].data_ptr() == a[0].data_ptr()
     assert _replay(step).recording is not None
+
+
+def test_calls_with_other_shapes_and_types_than_the_recorded_ones():
+    step = jp.mpmd_jit_by_yield(_chain, _mesh())
+    w = torch.randn(64, 64, device="cuda") / 8
+    x = torch.randn(32, 64, device="cuda")
+    step(x, w)
+    compiled = next(iter(step._cache.values()))
+    for _ in range(4):
+        compiled(x, w)
+    assert compiled._replay.recording is not None
+    for dtype, rows in ((torch.float32, 1), (torch.float64, 32), (torch.float32, 48)):
+        y, v = torch.randn(rows, 64, dtype=dtype, device="cuda"), w.to(dtype)
+        got = _tensors(compiled(y, v))
+        for t, r in zip(got, _chain_eager(y, v)):
+            assert t.shape == r.shape and t.dtype == r.dtype
+            torch.testing.assert_close(t, r, rtol=1e-4, atol=1e-4)
