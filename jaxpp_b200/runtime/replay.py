@@ -29,7 +29,8 @@ from .. import fault
 FREE_BYTES, BYTES_PER_OP, MAX_BYTES = 64 << 20, 1 << 20, 256 << 20
 MIN_OPS = 8
 MAX_POOL_BYTES = 512 << 20       # memory that one recording may keep for its intermediate values
-TOTAL_POOL_BYTES = 1 << 30       # and all recordings of the process together
+TOTAL_POOL_BYTES = 1 << 30       # what all recordings of the process keep together, their copies of the inputs included;
+                                 # programs that come when it is used up run op by op
 EAGER_CALLS = 2                  # calls that run op by op first: allocator, kernels and workspaces are warm, and a
                                  # program that is called once or twice is never recorded
 
@@ -107,6 +108,10 @@ def _copy_all(dst: list, src: list) -> None:
         torch._foreach_copy_(d, s)
 
 
+def _input_bytes(inputs: Sequence) -> int:
+    return sum(x.nbytes for x in inputs if x is not None)
+
+
 class _Recording:
     def __init__(self, prog: Program, inputs: Sequence, device: torch.device, execute):
         from ..ops import native
@@ -117,7 +122,6 @@ class _Recording:
         self.stream = torch.cuda.Stream(device)
         self.graph = torch.cuda.CUDAGraph()
         self.done = torch.cuda.Event()
-        before = torch.cuda.memory_reserved(device)
         launches = native.LAUNCHES[0]
         versions = [None if s is None else s._version for s in self.static]
         self.stream.wait_stream(torch.cuda.current_stream(device))
@@ -139,7 +143,9 @@ class _Recording:
                 gc.enable()
         self.launches = native.LAUNCHES[0] - launches
         native.LAUNCHES[0] = launches
-        self.pool_bytes = max(0, torch.cuda.memory_reserved(device) - before)
+        # the graph's own segments: other threads allocate meanwhile
+        self.pool_bytes = sum(seg["total_size"] for seg in torch.cuda.memory_snapshot(mempool_id=self.graph.pool(), include_traces=False))
+        self.kept_bytes = self.pool_bytes + _input_bytes(self.static)
         # (every static tensor has a storage of its own)
         self.written = [k for k, s in enumerate(self.static)
                         if s is not None and (s.untyped_storage().data_ptr() in written or s._version != versions[k])]
@@ -246,10 +252,11 @@ class StepReplay:
             return rec.run(inputs)
 
     def _record(self, inputs, device, execute) -> _Recording | None:
+        most = MAX_POOL_BYTES + _input_bytes(inputs)
         with _pool_lock:
-            if _pool_bytes[0] + MAX_POOL_BYTES > TOTAL_POOL_BYTES:
+            if _pool_bytes[0] + most > TOTAL_POOL_BYTES:
                 return None
-            _pool_bytes[0] += MAX_POOL_BYTES      # reserved until the size is known
+            _pool_bytes[0] += most      # reserved until the size is known
         rec = None
         try:
             rec = _Recording(self.prog, inputs, device, execute)
@@ -258,7 +265,7 @@ class StepReplay:
             logger.info("step is not replayed as a CUDA graph: %s", e)
         keep = rec is not None and rec.pool_bytes <= MAX_POOL_BYTES
         with _pool_lock:
-            _pool_bytes[0] += (rec.pool_bytes if keep else 0) - MAX_POOL_BYTES
+            _pool_bytes[0] += (rec.kept_bytes if keep else 0) - most
         if not keep:
             self.ok = False
             if rec is not None:
@@ -270,7 +277,7 @@ class StepReplay:
         rec, self.recording = self.recording, None
         if rec is not None:
             with _pool_lock:
-                _pool_bytes[0] -= rec.pool_bytes
+                _pool_bytes[0] -= rec.kept_bytes
             rec.release()
 
     def __del__(self):

@@ -1,4 +1,5 @@
 """Steps replayed as CUDA graphs against the same steps run op by op: same bits, other buffers on every call."""
+import gc
 import threading
 
 import pytest
@@ -9,6 +10,7 @@ import jaxpp_b200 as jp
 from jaxpp_b200.models import lm_trainer as lt
 from jaxpp_b200.models import transformer as tf
 from jaxpp_b200.ops import core as ops
+from jaxpp_b200.runtime import replay
 from jaxpp_b200.utils import config
 
 pytestmark = pytest.mark.gpu
@@ -187,3 +189,24 @@ def test_calls_with_other_shapes_and_types_than_the_recorded_ones():
         for t, r in zip(got, _chain_eager(y, v)):
             assert t.shape == r.shape and t.dtype == r.dtype
             torch.testing.assert_close(t, r, rtol=1e-4, atol=1e-4)
+
+
+def test_memory_of_all_recordings_is_bounded_with_their_inputs(monkeypatch):
+    """One program per shape, 65 MB of inputs each: the limit counts the copies of the inputs and is given back."""
+    gc.collect()
+    before, limit = replay._pool_bytes[0], replay.MAX_POOL_BYTES + (264 << 20)
+    monkeypatch.setattr(replay, "TOTAL_POOL_BYTES", before + limit)
+    step = jp.mpmd_jit_by_yield(_chain, _mesh())
+    w = torch.randn(4096, 4096, device="cuda") / 64
+    for rows in range(8, 80, 8):
+        x = torch.randn(rows, 4096, device="cuda")
+        for _ in range(4):
+            got = _tensors(step(x, w))
+        for t, r in zip(got, _chain_eager(x, w)):
+            torch.testing.assert_close(t, r, rtol=1e-3, atol=1e-3)
+    recs = [c._replay.recording for c in step._cache.values() if c._replay.recording is not None]
+    copies, kept = sum(s.nbytes for rec in recs for s in rec.static), replay._pool_bytes[0] - before
+    assert recs and copies < kept <= limit and len(recs) < 9
+    del recs, step, got
+    gc.collect()
+    assert replay._pool_bytes[0] == before
