@@ -219,8 +219,8 @@ class StepReplay:
         from . import executor
 
         if self.ok is None:
-            self.ok = device.type == "cuda" and config.step_graphs.value and _program_ok(self.prog)
-        if not self.ok or executor._TIMES or optimes.ACTIVE[0] or fault._PLAN[0] is not None or config.nvtx_ranges.value:
+            self.ok = device.type == "cuda" and _program_ok(self.prog)
+        if not self.ok or not config.step_graphs.value or executor._TIMES or optimes.ACTIVE[0] or fault._PLAN[0] is not None or config.nvtx_ranges.value:
             return False
         if os.environ.get("JAXPP_B200_TRACK_LIVE_BYTES") == "1" or torch.cuda.current_device() != (device.index or 0):
             return False

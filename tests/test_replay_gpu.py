@@ -210,3 +210,23 @@ def test_memory_of_all_recordings_is_bounded_with_their_inputs(monkeypatch):
     del recs, step, got
     gc.collect()
     assert replay._pool_bytes[0] == before
+
+
+def test_the_flag_holds_for_each_call():
+    w, x = torch.randn(64, 64, device="cuda") / 8, torch.randn(32, 64, device="cuda")
+    step = jp.mpmd_jit_by_yield(_chain, _mesh())
+    for on, recorded in ((True, False), (True, False), (False, False), (False, False), (True, True)):
+        with config.step_graphs.set(on):
+            step(x, w)
+        assert (_replay(step).recording is not None) == recorded
+    replays, run = [0], _replay(step).recording.run
+    _replay(step).recording.run = lambda inputs: (replays.__setitem__(0, replays[0] + 1), run(inputs))[1]
+    with config.step_graphs.set(False):
+        step(x, w)
+    assert replays[0] == 0
+    late = jp.mpmd_jit_by_yield(_chain, _mesh())
+    with config.step_graphs.set(False):      # a warm-up without graphs
+        late(x, w)
+    for _ in range(3):
+        late(x, w)
+    assert _replay(late).recording is not None
