@@ -45,8 +45,9 @@ _IDENTITY_TARGETS = {torch.ops.aten.detach.default, torch.ops.aten.alias.default
 class TaskCode:
     """Source text plus the tables it refers to; ``bind(device)`` gives the callable."""
 
-    def __init__(self, name: str, src: str, targets: list, consts: list, n_in: int, n_out: int, sink_outputs=()):
+    def __init__(self, name: str, src: str, targets: list, consts: list, n_in: int, n_out: int, sink_outputs=(), n_ops: int = 0):
         self.name, self.src, self.targets, self.consts, self.n_in, self.n_out = name, src, targets, consts, n_in, n_out
+        self.n_ops = n_ops      # calls of ops in one run, each at least one kernel launch
         # output positions produced by a weight-gradient op and by nothing else: ``run(args, sink)`` accepts an
         # accumulator for them (see ops/sink.py)
         self.sink_outputs = tuple(sink_outputs)
@@ -144,6 +145,7 @@ def generate(name: str, nodes: Sequence[fx.Node], inputs: Sequence[Any], outputs
     for j, k in enumerate(outputs):
         out_index.setdefault(k, []).append(j)
     sink_outputs: list[int] = []
+    n_ops = 0
 
     pre_free = [names[k] for k in inputs if last_use.get(k) == -1]
     if pre_free:
@@ -167,6 +169,7 @@ def generate(name: str, nodes: Sequence[fx.Node], inputs: Sequence[Any], outputs
                 # an alias of its operand: tasks are functional, so the operand itself serves
                 lines.append(f"    {var} = {aref(n.args[0], m)}")
             else:
+                n_ops += 1
                 parts = [aref(a, m) for a in n.args]
                 parts += [f"{kw}={aref(v, m)}" for kw, v in n.kwargs.items()]
                 if n.target in sinkable and k not in last_use and len(out_index.get(k, ())) == 1:
@@ -188,7 +191,7 @@ def generate(name: str, nodes: Sequence[fx.Node], inputs: Sequence[Any], outputs
 
     lines.append(f"    return [{', '.join(names[k] for k in outputs)}]")
     src = "def run(args, sink=None):\n" + "\n".join(lines) + "\n"
-    return TaskCode(name, src, targets, consts.items, len(inputs), len(outputs), sink_outputs)
+    return TaskCode(name, src, targets, consts.items, len(inputs), len(outputs), sink_outputs, n_ops)
 
 
 class CodeCache:

@@ -73,7 +73,7 @@ def _program_ok(prog: Program) -> bool:
                 return False
             if any(isinstance(c, torch.Tensor) for c in ins.code.consts):     # copied from the host on every run
                 return False
-            ops += ins.code.src.count(" = D[") + ins.code.src.count(" = T[") + ins.code.src.count(" = WG(")
+            ops += ins.code.n_ops
         elif not isinstance(ins, (Slice, Accum, Delete, SendDone)):
             return False
     in_bytes = sum(prog.values[vid].nbytes for vid, ranks in prog.inputs if ranks)

@@ -701,3 +701,23 @@ def test_force_mpmdify_with_cross_rank_collectives_and_a_failing_rank():
                 f(params, batch)
         finally:
             fault.set_fault_plan(None)
+
+
+def test_task_code_counts_its_ops_whatever_its_source_looks_like():
+    """Which steps are recorded as graphs goes by the number of ops; it must not hang on how the generated text is laid out."""
+    from jaxpp_b200.runtime import replay
+
+    def step(x, w):
+        y = x
+        for _ in range(6):
+            y = torch.tanh(y @ w) + x
+        return jp.mark_stage_end((y, y.sum(0)))
+
+    f = jp.mpmd_jit_by_yield(step, cpu_mesh(1))
+    f(torch.randn(4, 8), torch.randn(8, 8))
+    prog = next(iter(f._cache.values())).program
+    codes = [ins.code for ins in prog.instrs if isinstance(ins, RunTask)]
+    for code in codes:
+        code.src = code.src.replace(" = ", "  =  ")
+    assert replay._program_ok(prog)
+    assert sum(code.n_ops for code in codes) == 6 * 3 + 1
