@@ -173,6 +173,7 @@ class _Recording:
                 n = len(self.results)
                 self.results.append(t)
             self.outputs.append(("out", rank, n))
+        self.done.record(torch.cuda.current_stream(device))     # the first copies into the buffers
 
     def covers(self, inputs: Sequence) -> bool:
         """A compiled step runs on whatever tensors it is called with; the recording is one of these shapes and dtypes."""
@@ -184,16 +185,18 @@ class _Recording:
 
         stream = torch.cuda.current_stream(self.device)
         stream.wait_event(self.done)       # the buffers may still be in use by a replay on another stream
+        fresh = [torch.empty_like(t) for t in self.results]     # (if there is no memory for them, nothing has run yet)
         live = [(s, x) for s, x in zip(self.static, inputs) if s is not None]
-        _copy_all([s for s, _ in live], [x.detach() for _, x in live])
-        self.graph.replay()
-        native.LAUNCHES[0] += self.launches
-        fresh = [torch.empty_like(t) for t in self.results]
-        _copy_all(fresh, self.results)
-        if self.written:
-            # (.data: like the kernels' own in-place updates, this does not touch autograd's version counters)
-            _copy_all([inputs[k].data for k in self.written], [self.static[k] for k in self.written])
-        self.done.record(stream)
+        try:
+            _copy_all([s for s, _ in live], [x.detach() for _, x in live])
+            self.graph.replay()
+            native.LAUNCHES[0] += self.launches
+            _copy_all(fresh, self.results)
+            if self.written:
+                # (.data: like the kernels' own in-place updates, this does not touch autograd's version counters)
+                _copy_all([inputs[k].data for k in self.written], [self.static[k] for k in self.written])
+        finally:
+            self.done.record(stream)       # whatever is in flight uses the buffers, also after an error
         return [o[1] if o[0] == "c" else {o[1]: inputs[o[2]] if o[0] == "in" else fresh[o[2]]} for o in self.outputs]
 
     def release(self) -> None:
