@@ -331,6 +331,16 @@ def test_load_balancing_loss_repeats_and_is_summed_in_trees(native, T, E, k):
     assert abs(aux.double() - want) <= steps * 2.0 ** -24 * want
 
 
+@pytest.mark.parametrize("rows", [128, 250, 256])
+def test_parameter_sums_are_added_in_trees(native, rows):
+    """One large row among small ones, each row a partial sum of its own: at most 2 + 2 + 5 additions (within a thread, of its
+    four sums, between 32 threads) have the large value as an operand, and each loses at most half a unit in its last place."""
+    x = torch.full((rows, 64), 0.125, device="cuda")
+    x[0] = 2.0 ** 24
+    want = 2.0 ** 24 + (rows - 1) / 8
+    assert ((native.colsum(x).double() - want).abs() <= 9 * 1.0).all()
+
+
 @pytest.mark.parametrize("layer", [False, True])
 @pytest.mark.parametrize("rows,H", [(2400, 1600), (9500, 256), (4737, 4096), (300, 8192)])
 def test_norm_backward_over_many_rows(native, layer, rows, H):
