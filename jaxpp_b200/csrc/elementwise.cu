@@ -890,14 +890,17 @@ JPB_API int jpb_norm_fwd(int layer, int dt, const void* x, const void* w, const 
 }
 
 // CTAs of the norm backward: as many as are resident at once (its 128 registers per thread leave room for 512 threads per
-// SM), since every CTA leaves 2 H partial sums behind and a second wave would be a ragged one.  A row of 1600 bf16 is a CTA
-// of 128 threads, and two of those per SM left the memory system idle: 16384 rows took 139 us, with four 85, with eight, half of them waiting, 101;
-// rows of 4096 (256 threads) take 42 us with two per SM and 50 with up to four.  Few rows: two per SM.
+// SM), since every CTA leaves 2 H partial sums behind and a second wave would be a ragged one -- but not so many that a CTA
+// gets fewer than six rows, where uneven shares and the sum over the partial rows cost more than the extra loads in flight
+// gain.  bf16, operands in L2 / in HBM with the residual gradient added: 16384 rows of 1600 (CTAs of 128 threads) 67 / 77 us
+// with two CTAs per SM, 47 / 56 with four, 54 / 62 with eight, half of them waiting; 3000 of 2048 16.9 / 22.0 with two, 19.6 /
+// 21.5 with four; 6000 of 1024 (64 threads) 19.5 / 32.3 with two, 18.6 / 24.7 with four, 21.0 / 24.0 with eight; rows of 4096
+// (256 threads) 31 / 38 with two per SM and 39 / 44 with four.
 static int norm_bwd_grid(int rows, int H, int vn) {
   const int threads = norm_threads(H, vn, NORM_BWD_VECS);
-  const int per_sm = threads > 128 ? 2 : 512 / threads < 8 ? 512 / threads : 8;
-  const int full = sm_count() * per_sm;
-  const int grid = rows >= 4 * full ? full : sm_count() * 2;
+  int per_sm = threads > 128 ? 2 : 512 / threads < 8 ? 512 / threads : 8;
+  while (per_sm > 2 && rows < 6 * sm_count() * per_sm) per_sm /= 2;
+  const int grid = sm_count() * per_sm;
   return rows < grid ? rows : grid;
 }
 

@@ -549,6 +549,21 @@ def test_flash_attention_at_block_edges(native, B, Sq, Sk, H, Hkv, causal, D):
     assert native.read_status(clear=False) == 0
 
 
+@pytest.mark.parametrize("rows,H,per_sm", [(3000, 2048, 2), (6000, 1024, 4), (7200, 1024, 8), (3600, 1600, 4), (9000, 4096, 2)])
+def test_norm_backward_gives_every_cta_six_rows(native, rows, H, per_sm):
+    """(the numbers of rows are for 148 SMs)  The grid shows in the scratch, 2 H sums per CTA; the sums against 64 bits, rounded
+    to bf16 once."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    if sms == 148:
+        assert native.load().jpb_norm_bwd_scratch_elems(rows, H) == max(sms * per_sm, min(rows, sms * 2)) * 2 * H
+    x, w, dy = rnd(rows, H, seed=1), rnd(H, seed=2), rnd(rows, H, seed=3)
+    rstd = (x.double().pow(2).mean(-1) + 1e-5).rsqrt().float()
+    want = (dy.double() * x.double() * rstd.double()[:, None]).sum(0)
+    dw = native.rmsnorm_bwd(dy, x, w, rstd)[1]
+    slack = rows * 2.0 ** -23 * (dy.double() * x.double() * rstd.double()[:, None]).abs().sum(0)
+    assert ((dw.double() - want).abs() <= 2.0 ** -8 * want.abs() + slack).all()
+
+
 @pytest.mark.parametrize("B,Sq,Sk,H,Hkv,D,causal", ATTN_CASES)
 def test_flash_attention_forward_backward(native, B, Sq, Sk, H, Hkv, D, causal):
     from jaxpp_b200.ops import attention as att
