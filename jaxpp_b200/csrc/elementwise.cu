@@ -1166,7 +1166,9 @@ JPB_API int jpb_adamw(int grad_dt, int out_dt, const float* p, const void* g, co
   for (const void* x : {(const void*)p, g, (const void*)m, (const void*)v, (const void*)p_out, (const void*)m_out, (const void*)v_out,
                         (const void*)lp_out})
     at |= reinterpret_cast<uintptr_t>(x);
-  const bool wide = (at & 15) == 0;
+  // One element per thread keeps more threads busy in small tensors: 1000 elements 1.37 us against 1.53, 65536 1.78 against
+  // 1.84, 131072 1.92 either way, 262144 2.39 against 2.23, 4194304 12.5 against 11.0.
+  const bool wide = (at & 15) == 0 && n >= 1 << 17;
   const int grid = ew_grid(wide ? size_t(n + 3) / 4 : size_t(n), 256);
 #define ADAMW(G, O)                                                                                                                \
   (wide ? adamw_kernel<G, O, 4><<<grid, 256, 0, STREAM>>>(p, (const G*)g, m, v, (const int64_t*)step, clip, p_out, m_out, v_out,    \

@@ -399,6 +399,17 @@ def test_adamw_with_clip_coefficient(native, n, offset, gdt):
         assert torch.equal(got[3], got[0].to(torch.bfloat16))
 
 
+@pytest.mark.parametrize("n", [(1 << 17) - 1, 1 << 17, (1 << 17) + 3])
+def test_adamw_gives_the_same_bits_at_either_width(native, n):
+    """Four elements per access from 2^17 elements on, one below and where a tensor is not on a 16-byte boundary."""
+    args = (torch.tensor(7, device="cuda"), 1e-2, 0.9, 0.95, 1e-8, 0.1, 0.5, torch.bfloat16)
+    results = []
+    for offset in (0, 1):
+        p, g, m, v = (torch.cat([torch.zeros(offset, device="cuda"), rnd(n, dtype=torch.float32, seed=s)])[offset:] for s in (1, 2, 3, 4))
+        results.append(native.adamw(p, g, m, v.abs_(), *args, None, True))
+    assert all(torch.equal(a, b) for a, b in zip(*results))
+
+
 @pytest.mark.parametrize("vocab,d,n", [(8200, 1032, 700), (9000, 1024, 1), (70000, 128, 3000)])
 def test_embedding_gradient_of_a_bf16_table(native, vocab, d, n):
     """Lists of tokens per id: ids that occur once, never and hundreds of times, more than one CTA per row, out of range;
