@@ -596,12 +596,20 @@ __global__ void embedding_bwd_kernel(const T* __restrict__ dy, const int64_t* __
 // The same gradient for a bf16 table, without an fp32 staging table of its size: the tokens of every id are collected in a
 // list (three passes over the ids), and the CTAs of an id's first token add up its rows in fp32 registers and write, or add
 // to, the table's row once.  Bound by the rows of dy and the touched rows of the table (32000 x 8192, 4096 tokens: 67 MB
-// each way; clearing, scattering into and casting an fp32 table moved 2.7 GB, 1.07 ms).
+// each way; clearing, scattering into and casting an fp32 table moved 2.7 GB, 1.07 ms) while no id dominates.  A long list
+// (padding can be most of a batch) is cut into segments of EMB_SEG rows, the last up to twice as long, each added up by CTAs
+// of its own into an fp32 row; the CTA that finishes last adds these in order.
+// 32000 x 8192, 16384 tokens of one id: 268 us, with one CTA per 1024 columns 6220; 16384 different ones: 196 us either way,
+// which takes 16 CTAs per SM (32 registers): at 40 registers it is 221.
+constexpr int EMB_SEG = 64;
 struct EmbLists {
   int* count;    // [vocab] tokens per id, zero on entry; count[vocab]: tokens placed so far
+  int* done;     // [n_tok / EMB_SEG + 1][gridDim.y] finished segments of a long list, by the place of its first segment, zero on entry
   int* base;     // [vocab] start of an id's list (of ids that occur)
   int* rank;     // [n_tok] position of a token in its id's list, -1: id out of range
   int* list;     // [n_tok]
+  float* part;   // [n_tok / EMB_SEG + 1][d] sums of the segments of long lists: segments start at least EMB_SEG apart, and
+                 // the one that starts at `first` has row first / EMB_SEG
 };
 __global__ void emb_count_kernel(const int64_t* __restrict__ ids, EmbLists l, int n_tok, int vocab) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -620,26 +628,67 @@ __global__ void emb_list_kernel(const int64_t* __restrict__ ids, EmbLists l, int
   l.list[l.base[ids[t]] + l.rank[t]] = t;
 }
 constexpr int EMB_THREADS = 128;
-__global__ void __launch_bounds__(EMB_THREADS) emb_sum_kernel(const __nv_bfloat16* __restrict__ dy, const int64_t* __restrict__ ids, EmbLists l,
+__global__ void __launch_bounds__(EMB_THREADS, 16) emb_sum_kernel(const __nv_bfloat16* __restrict__ dy, const int64_t* __restrict__ ids, EmbLists l,
                                                               __nv_bfloat16* __restrict__ table, int d, int accumulate) {
   constexpr int VN = Vec<__nv_bfloat16>::N;
+  static_assert(VN == 8 && 2 * EMB_SEG <= EMB_THREADS, "");
+  __shared__ int rows[2 * EMB_SEG];
+  __shared__ bool last;
   const int t = blockIdx.x;
-  if (l.rank[t] != 0) return;
+  const int rank = l.rank[t];
+  if (rank < 0 || rank % EMB_SEG) return;     // (all of these are uniform in the CTA)
   const int64_t id = ids[t];
-  const int n = l.count[id];
-  const int* list = l.list + l.base[id];
+  const int n = l.count[id], segs = n < 2 * EMB_SEG ? 1 : n / EMB_SEG, seg = rank / EMB_SEG;
+  if (seg >= segs) return;
+  const int base = l.base[id], first = base + seg * EMB_SEG;
+  const int len = seg + 1 < segs ? EMB_SEG : n - seg * EMB_SEG;
   const int c = (blockIdx.y * EMB_THREADS + threadIdx.x) * VN;
-  if (c >= d) return;
+  const bool in = c < d;
   float acc[VN];
+  if (n == 1) {                               // most ids of a batch of different tokens: nothing to look up
+    if (!in) return;
+    Vec<__nv_bfloat16> v; v.load(dy + size_t(t) * d + c);
+    v.to_float(acc);
+  } else {
+    if (threadIdx.x < len) rows[threadIdx.x] = l.list[first + threadIdx.x];
+    __syncthreads();
 #pragma unroll
-  for (int j = 0; j < VN; ++j) acc[j] = 0.f;
+    for (int j = 0; j < VN; ++j) acc[j] = 0.f;
+    if (in) {
 #pragma unroll 4
-  for (int i = 0; i < n; ++i) {
-    Vec<__nv_bfloat16> v; v.load(dy + size_t(list[i]) * d + c);
-    float f[VN]; v.to_float(f);
+      for (int i = 0; i < len; ++i) {
+        Vec<__nv_bfloat16> v; v.load(dy + size_t(rows[i]) * d + c);
+        float f[VN]; v.to_float(f);
 #pragma unroll
-    for (int j = 0; j < VN; ++j) acc[j] += f[j];
+        for (int j = 0; j < VN; ++j) acc[j] += f[j];
+      }
+    }
   }
+  if (segs > 1) {
+    if (in) {
+      float4* p = reinterpret_cast<float4*>(l.part + size_t(first / EMB_SEG) * d + c);
+      p[0] = make_float4(acc[0], acc[1], acc[2], acc[3]);
+      p[1] = make_float4(acc[4], acc[5], acc[6], acc[7]);
+    }
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(&l.done[size_t(base / EMB_SEG) * gridDim.y + blockIdx.y], 1) == segs - 1;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+#pragma unroll
+    for (int j = 0; j < VN; ++j) acc[j] = 0.f;
+    if (in) {
+#pragma unroll 1
+      for (int i = 0; i < segs; ++i) {
+        const float4* p = reinterpret_cast<const float4*>(l.part + size_t((base + i * EMB_SEG) / EMB_SEG) * d + c);
+        const float4 a = __ldcg(p), b = __ldcg(p + 1);
+        acc[0] += a.x; acc[1] += a.y; acc[2] += a.z; acc[3] += a.w;
+        acc[4] += b.x; acc[5] += b.y; acc[6] += b.z; acc[7] += b.w;
+      }
+    }
+  }
+  if (!in) return;
   __nv_bfloat16* row = table + size_t(id) * d + c;
   Vec<__nv_bfloat16> o; o.from_float(acc);
   if (accumulate) {   // the sum is rounded before it is added, as a gradient tensor of its own would be
@@ -1086,26 +1135,42 @@ JPB_API int jpb_embedding_bwd_acc(int dt, const void* dy, const long long* ids, 
   });
 }
 
-// Gradient of a bf16 table [vocab, d] from bf16 rows, cleared first or added to.  `scratch`: 2 * vocab + 1 + 2 * n_tok ints.
-JPB_API int jpb_embedding_bwd_bf16(const void* dy, const long long* ids, void* table, int* scratch, int n_tok, int d, int vocab,
+static int emb_chunks(int d) {   // CTAs along a row
+  const int per = EMB_THREADS * Vec<__nv_bfloat16>::N;
+  return (d + per - 1) / per;
+}
+static size_t emb_ints(int n_tok, int d, int vocab) {   // of EmbLists, up to a 16-byte boundary
+  return (2 * size_t(vocab) + 1 + size_t(n_tok / EMB_SEG + 1) * emb_chunks(d) + 2 * size_t(n_tok) + 3) & ~size_t(3);
+}
+JPB_API long long jpb_embedding_bwd_bf16_scratch_bytes(int n_tok, int d, int vocab) {
+  return (long long)(emb_ints(n_tok, d, vocab) * 4 + (n_tok < 2 * EMB_SEG ? 0 : size_t(n_tok / EMB_SEG + 1) * d * 4));
+}
+
+// Gradient of a bf16 table [vocab, d] from bf16 rows, cleared first or added to.  `scratch`:
+// jpb_embedding_bwd_bf16_scratch_bytes(), on a 16-byte boundary.
+JPB_API int jpb_embedding_bwd_bf16(const void* dy, const long long* ids, void* table, void* scratch, int n_tok, int d, int vocab,
                                    int accumulate, void* stream) {
-  if (d % Vec<__nv_bfloat16>::N || (reinterpret_cast<uintptr_t>(table) & 15)) return -int(JPB_ERR_BAD_ARGUMENT);
+  if (d % Vec<__nv_bfloat16>::N || ((reinterpret_cast<uintptr_t>(table) | reinterpret_cast<uintptr_t>(scratch)) & 15))
+    return -int(JPB_ERR_BAD_ARGUMENT);
   if (!accumulate) cudaMemsetAsync(table, 0, size_t(vocab) * d * sizeof(__nv_bfloat16), STREAM);
   if (n_tok <= 0) return LAST_ERR;
+  const int chunks = emb_chunks(d);
+  const size_t n_done = size_t(n_tok / EMB_SEG + 1) * chunks;
   EmbLists l;
-  l.count = scratch;
-  l.base = scratch + vocab + 1;
+  l.count = static_cast<int*>(scratch);
+  l.done = l.count + vocab + 1;
+  l.base = l.done + n_done;
   l.rank = l.base + vocab;
   l.list = l.rank + n_tok;
-  cudaMemsetAsync(l.count, 0, size_t(vocab + 1) * sizeof(int), STREAM);
+  l.part = reinterpret_cast<float*>(static_cast<int*>(scratch) + emb_ints(n_tok, d, vocab));
+  cudaMemsetAsync(l.count, 0, (size_t(vocab) + 1 + n_done) * sizeof(int), STREAM);
   const int64_t* id = reinterpret_cast<const int64_t*>(ids);
   const int blocks = (n_tok + 255) / 256;
   emb_count_kernel<<<blocks, 256, 0, STREAM>>>(id, l, n_tok, vocab);
   emb_base_kernel<<<blocks, 256, 0, STREAM>>>(id, l, n_tok, vocab);
   emb_list_kernel<<<blocks, 256, 0, STREAM>>>(id, l, n_tok);
-  const int per = EMB_THREADS * Vec<__nv_bfloat16>::N;
-  emb_sum_kernel<<<dim3(n_tok, (d + per - 1) / per), EMB_THREADS, 0, STREAM>>>(static_cast<const __nv_bfloat16*>(dy), id, l,
-                                                                               static_cast<__nv_bfloat16*>(table), d, accumulate);
+  emb_sum_kernel<<<dim3(n_tok, chunks), EMB_THREADS, 0, STREAM>>>(static_cast<const __nv_bfloat16*>(dy), id, l,
+                                                                  static_cast<__nv_bfloat16*>(table), d, accumulate);
   return LAST_ERR;
 }
 

@@ -499,7 +499,9 @@ def embedding_bwd(dy, ids, vocab, out_dtype=None, out: Optional[torch.Tensor] = 
         if not table.is_contiguous():
             raise NativeError("embedding_bwd accumulates into a contiguous table")
         n = ids.numel()
-        scratch = torch.empty(2 * vocab + 1 + 2 * n, dtype=torch.int32, device=dy.device)
+        lib.jpb_embedding_bwd_bf16_scratch_bytes.argtypes = [_c_int, _c_int, _c_int]
+        lib.jpb_embedding_bwd_bf16_scratch_bytes.restype = _c_ll
+        scratch = torch.empty(lib.jpb_embedding_bwd_bf16_scratch_bytes(n, d, vocab), dtype=torch.uint8, device=dy.device)
         _check(lib.jpb_embedding_bwd_bf16(dy.data_ptr(), ids.data_ptr(), table.data_ptr(), scratch.data_ptr(), n, d, vocab,
                                           int(accumulate), _stream()), "embedding_bwd", 4)
         return table

@@ -446,6 +446,47 @@ def test_dropout_matches_counter_based_reference(native, dtype):
     assert abs(drop - 0.3) < 5e-3
 
 
+@pytest.mark.parametrize("n,d", [(127, 8200), (128, 8200), (129, 1000), (192, 1032), (20000, 520)])
+def test_embedding_gradient_of_long_token_lists(native, n, d):
+    """Lists at the edges of the segments that they are cut into, two long ones behind each other and short ones between."""
+    vocab = 1100
+    ids = torch.randint(0, 64, (n + 40,), generator=torch.Generator().manual_seed(4))
+    ids[20:20 + n] = 70
+    ids = torch.cat([ids, torch.full((150,), 71), torch.full((5,), -1), torch.full((300,), 72)]).cuda()
+    dy = rnd(ids.numel(), d, seed=8)
+    ok = ids >= 0
+    want, size = (torch.zeros(vocab, d, dtype=torch.float64, device="cuda").index_add_(0, ids[ok], t) for t in (dy[ok].double(), dy[ok].double().abs()))
+    for out in (torch.full((vocab, d), float("nan"), dtype=torch.bfloat16, device="cuda"), torch.ones(vocab, d, dtype=torch.bfloat16, device="cuda")):
+        accumulate = not bool(out.isnan().any())
+        native.embedding_bwd(dy, ids, vocab, out=out, accumulate=accumulate)
+        # chains of at most 128 rows and n / 64 segments in fp32, rounded to bf16 (and once more where it is added to 1)
+        slack = (128 + n / 64) * 2.0 ** -24 * size + 2.0 ** -8 * (want.abs() + accumulate * (1 + want).abs())
+        assert ((out.double() - want - float(accumulate)).abs() <= slack).all()
+
+
+def test_embedding_gradient_does_not_wait_for_a_dominant_token(native):
+    """A batch that is 90 % padding costs about what a batch of different tokens does (measured 1.6 times that; as one
+    chain of rows it took fifty times as long)."""
+    vocab, d, n = 32000, 4096, 16384
+    ids = torch.randint(0, vocab, (n,), generator=torch.Generator().manual_seed(4)).cuda()
+    padded = ids.clone()
+    padded[n // 10:] = 3
+    dy = rnd(n, d, seed=8)
+
+    def best(tokens):
+        times = []
+        for _ in range(6):
+            start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            start.record()
+            native.embedding_bwd(dy, tokens, vocab)
+            end.record()
+            end.synchronize()
+            times.append(start.elapsed_time(end))
+        return min(times[1:])
+
+    assert best(padded) < 3 * best(ids)
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_embedding_and_cross_entropy(native, dtype):
     from jaxpp_b200.ops import core as ops
