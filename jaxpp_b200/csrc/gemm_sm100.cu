@@ -637,26 +637,59 @@ enum Form { PAIR256, PAIR128, ONE128, ONE64, FORMS };
 struct Choice {
   int form, split;
 };
-static Choice choose(const GemmParams& p) {
-  const int sms = num_sms();
+struct Resident {      // how many fit on the device at once: CTAs, clusters of two and of four
+  int ctas, pairs, quads;
+};
+static Choice choose(long long batch, int M, int N, int K, bool counted, const Resident& res) {
   constexpr int tm[FORMS] = {256, 256, 128, 128}, tn[FORMS] = {256, 128, 128, 64}, ctas[FORMS] = {2, 2, 1, 1};
   constexpr double start[FORMS] = {4.5, 3.5, 3.0, 2.5}, tile[FORMS] = {0.7, 0.7, 0.3, 0.2}, step[FORMS] = {0.37, 0.255, 0.35, 0.31};
-  const int k_blocks = (p.K + BK - 1) / BK;
+  const int k_blocks = (K + BK - 1) / BK;
   Choice best{PAIR256, 1};
   double best_t = 1e30;
   for (int f = 0; f < FORMS; ++f) {
-    const long long tiles = (long long)p.batch * ((p.M + tm[f] - 1) / tm[f]) * ((p.N + tn[f] - 1) / tn[f]);
-    const int slots = sms / ctas[f];
+    const long long tiles = batch * ((M + tm[f] - 1) / tm[f]) * ((N + tn[f] - 1) / tn[f]);
+    const int slots = ctas[f] == 2 ? res.pairs : res.ctas;
     const double waves = double((tiles + slots - 1) / slots);
     const double t = start[f] + waves * (tile[f] + k_blocks * step[f]);
     if (t < best_t) { best_t = t; best = {f, 1}; }
-    if (f != ONE64 || p.counts != nullptr) continue;
-    for (int split = 2; split <= 4 && tiles * split <= sms && k_blocks >= 8 * split; split *= 2) {
+    if (f != ONE64 || counted) continue;
+    // (only in one round: 33 clusters of four are resident, and 36 tiles in four parts each, 128 x 2304 x 4096, took 20.4 us in
+    // two rounds; in two parts they take 16.7)
+    for (int split = 2; split <= 4 && tiles <= (split == 2 ? res.pairs : res.quads) && k_blocks >= 8 * split; split *= 2) {
       const double ts = start[f] + 2.0 + tile[f] + (k_blocks / split) * step[f];
       if (ts < best_t) { best_t = ts; best = {f, split}; }
     }
   }
   return best;
+}
+
+// Clusters of `size` CTAs of this kernel that are resident at once.  148 SMs hold 74 pairs but only 33 clusters of four.
+template <int CG, int BN, bool SPLIT>
+static int resident_clusters(int size) {
+  auto kernel = gemm_bf16_kernel<CG, BN, SPLIT, false, false>;
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<CG, BN>::SMEM_BYTES) != cudaSuccess) return 0;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(num_sms() / size * size);
+  cfg.blockDim = dim3(GEMM_THREADS);
+  cfg.dynamicSmemBytes = Cfg<CG, BN>::SMEM_BYTES;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = size;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  int n = 0;
+  if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
+    cudaGetLastError();   // not an error of the launch that follows
+    n = 0;
+  }
+  const int whole = num_sms() / size;
+  return n > 0 && n < whole ? n : whole;
+}
+static const Resident& resident() {
+  static const Resident r = {num_sms(), resident_clusters<2, 256, false>(2), resident_clusters<1, 64, true>(4)};
+  return r;
 }
 
 template <int CG, int BN, bool SPLIT, bool A_MN, bool B_MN>
@@ -668,7 +701,7 @@ static int launch(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMa
   if (configured != cudaSuccess) return int(configured);
   const int ctas = SPLIT ? p.split : CG;
   const int tiles = p.tiles_m * p.tiles_n * p.batch;
-  const int slots = num_sms() / ctas;
+  const int slots = CG == 2 ? resident().pairs : num_sms() / ctas;
   const int clusters = SPLIT ? tiles : (tiles < slots ? tiles : slots);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(clusters * ctas);
@@ -721,7 +754,7 @@ static int gemm_entry(const void* A, const void* B, void* D, const void* bias, i
   p.M = M; p.N = N; p.K = K; p.ldd = ldd; p.out_fp32 = out_fp32; p.accumulate = accumulate;
   p.bias = bias; p.bias_fp32 = bias_fp32; p.D = D; p.status = jpb_status_device_ptr();
   p.counts = counts; p.seg_rows = seg_rows; p.segs = segs; p.count_k = count_k;
-  const Choice choice = choose(p);
+  const Choice choice = choose(batch, M, N, K, counts != nullptr, resident());
   const int tm = choice.form <= PAIR128 ? 256 : 128;
   const int tn = choice.form == PAIR256 ? 256 : choice.form == ONE64 ? 64 : 128;
   const int b_rows = choice.form == PAIR256 || choice.form == ONE128 ? 128 : 64;  // rows of B per CTA
@@ -756,6 +789,16 @@ static int gemm_entry(const void* A, const void* B, void* D, const void* bias, i
       if (choice.split > 1) return launch_layout<1, 64, true>(ma, mb, md, p, a_mn_major, b_mn_major, s);
       return launch_layout<1, 64, false>(ma, mb, md, p, a_mn_major, b_mn_major, s);
   }
+}
+
+// The form that `batch` products [M, K] x [K, N] take, and the parts of their reductions (times 16), on a device that holds
+// `ctas` CTAs, `pairs` clusters of two and `quads` of four at once (ctas = 0: this device).  Forms: 0 and 1 pairs of CTAs with
+// 256 and 128 columns, 2 and 3 single CTAs with 128 and 64.
+JPB_API int jpb_gemm_form(int batch, int M, int N, int K, int counted, int ctas, int pairs, int quads) {
+  const jpb::Resident res = ctas > 0 ? jpb::Resident{ctas, pairs, quads} : jpb::resident();
+  if (res.ctas <= 0 || res.pairs <= 0 || res.quads <= 0 || batch <= 0 || M <= 0 || N <= 0 || K <= 0) return -JPB_ERR_BAD_ARGUMENT;
+  const jpb::Choice c = jpb::choose(batch, M, N, K, counted != 0, res);
+  return c.form + 16 * c.split;
 }
 
 // A: [M,K] with lda (K-major) or stored as [K,M] with lda (MN-major); likewise B for [N,K] / [K,N].
