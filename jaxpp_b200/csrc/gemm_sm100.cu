@@ -4,8 +4,8 @@
 //   CG = 2  a pair of CTAs (one cluster, tcgen05 cta_group::2) shares a 256 x BN tile: each CTA holds its 128 rows of A
 //           and half of the BN rows of B per stage and 128 x BN of the accumulator, so an operand byte in shared memory
 //           feeds twice the products of a tile of one CTA;
-//   CG = 1  one CTA per 128 x BN tile, for outputs with too few tiles for the pairs; with SPLIT, a cluster of CTAs
-//           divides the reduction of one tile and adds the parts through distributed shared memory.
+//   CG = 1  one CTA per 128 x BN tile, for outputs with too few tiles for the pairs or with few rows; with SPLIT, a
+//           cluster of CTAs divides the reduction of one tile and adds the parts through distributed shared memory.
 // Warp 0 streams operand tiles into a shared-memory ring with TMA (128-byte swizzle), warp 1 (of the leader) issues
 // tcgen05.mma into one of two TMEM accumulators, warps 2-5 drain the other one with tcgen05.ld, so the epilogue of
 // tile i overlaps the main loop of tile i+1.  The epilogue (+ bias, or added onto an existing fp32 D) goes through
@@ -626,40 +626,60 @@ static int num_sms() {
   return n;
 }
 
-// Which form a product takes.  A launch takes about  start + waves x (tile + k blocks x step);  the constants are
-// microseconds, fitted to runs of every form from 256^3 to 4096 x 32000 x 4096: a step of a pair costs half as much per
-// product as that of a single CTA (4096 x 12288 x 4096: 269 us with 256 x 256 pairs, 341 with 256 x 128 pairs; 4096^3:
-// 100, 132 and, for single CTAs, 152 with 128 x 128 and 285 with 128 x 64; the 128 x 256 tiles of one CTA used before
-// 155), but a large tile starts and ends slowly and leaves SMs idle when there are few of them (256^3: 8.9 us against 7.4
-// with 128 x 64 tiles; 1024 x 1600 x 1600: 15 us against 12.5).  Reductions are divided only where that leaves no CTA
-// without an SM, and down to eight k blocks per part (77 x 4096 x 11008: 45 us whole, 31 us in two parts).
-enum Form { PAIR256, PAIR128, ONE128, ONE64, FORMS };
+// Which form a product takes.  A launch takes about
+//     start + sum over waves of max(main + k blocks x step, out) + out     microseconds,
+// a wave being as many tiles as there are CTAs (pairs, clusters) at a time and `out` the epilogue of a tile, which overlaps
+// the next tile's products.  A step is not shorter than its part of B takes from memory (with few rows of output the product
+// is a pass over B).  The constants were fitted to every form's time at 1410 products (outputs of 8 to 8192 rows and
+// 128 to 50304 columns, reductions of 8 to 28672, all three layouts, bf16 and accumulated fp32 results; A in L2, B and the
+// result taking turns through more memory than L2 holds).  The form with the least estimate is 0.4 % slower than the fastest
+// one on average, 31 % at worst (8 x 7776 x 432); without the terms for the epilogue and for B and without the third form
+// it was 7 to 12 % and up to three times.
+//   256 x 256 pairs       large outputs: 4096^3 100 us (128 columns 132, single CTAs of 128 columns 152)
+//   256 x 128 pairs       768 x 1024 x 28672: 102 us, single CTAs of 64 columns 116
+//   128 x 256, one CTA    one wave where narrower tiles need a second, and few rows of A, which every tile fetches again:
+//                         128 x 22016 x 4096 38 us, 128 columns 49; 8 x 32000 x 4096 53 us, 69; 384 x 11008 x 4096 36 us,
+//                         pairs 41
+//   128 x 128, 128 x 64   few tiles, and short reductions, whose time is the epilogue's: 768 x 256 x 1024 with 64 columns
+//                         8.3 us, 256 10.1
+//   divided reductions    cost 2 to 4 us of their own: 128 x 2304 x 4096 16.7 us in two parts, whole 23; in four 20.4, since
+//                         only 33 clusters of four CTAs are resident at once and its 36 tiles took two rounds
+enum Form { PAIR256, PAIR128, ONE256, ONE128, ONE64, FORMS };
 struct Choice {
   int form, split;
 };
 struct Resident {      // how many fit on the device at once: CTAs, clusters of two and of four
   int ctas, pairs, quads;
 };
-static Choice choose(long long batch, int M, int N, int K, bool counted, const Resident& res) {
-  constexpr int tm[FORMS] = {256, 256, 128, 128}, tn[FORMS] = {256, 128, 128, 64}, ctas[FORMS] = {2, 2, 1, 1};
-  constexpr double start[FORMS] = {4.5, 3.5, 3.0, 2.5}, tile[FORMS] = {0.7, 0.7, 0.3, 0.2}, step[FORMS] = {0.37, 0.255, 0.35, 0.31};
+static Choice choose(long long batch, int M, int N, int K, bool out_fp32, bool counted, const Resident& res) {
+  constexpr int tm[FORMS] = {256, 256, 128, 128, 128}, tn[FORMS] = {256, 128, 256, 128, 64};
+  constexpr double start[FORMS] = {3.0, 2.1, 2.5, 2.7, 2.9}, main[FORMS] = {0.6, 1.5, 1.1, 0.9, 0.9},
+                   step[FORMS] = {0.306, 0.253, 0.372, 0.277, 0.268}, out[FORMS] = {2.8, 2.2, 1.7, 1.1, 0.6};
+  constexpr double bytes_per_us = 5.4e6;   // B from memory, all CTAs together
+  const double out_scale = out_fp32 ? 1.4 : 1.0;
+  // few rows: every CTA asks for the same lines of A at the same time, the more often the narrower its tiles are
+  const double few_rows = M < 64 ? 0.037 * (64 - M) / 64 : 0.0;
   const int k_blocks = (K + BK - 1) / BK;
   Choice best{PAIR256, 1};
   double best_t = 1e30;
-  for (int f = 0; f < FORMS; ++f) {
-    const long long tiles = batch * ((M + tm[f] - 1) / tm[f]) * ((N + tn[f] - 1) / tn[f]);
-    const int slots = ctas[f] == 2 ? res.pairs : res.ctas;
-    const double waves = double((tiles + slots - 1) / slots);
-    const double t = start[f] + waves * (tile[f] + k_blocks * step[f]);
-    if (t < best_t) { best_t = t; best = {f, 1}; }
-    if (f != ONE64 || counted) continue;
-    // (only in one round: 33 clusters of four are resident, and 36 tiles in four parts each, 128 x 2304 x 4096, took 20.4 us in
-    // two rounds; in two parts they take 16.7)
-    for (int split = 2; split <= 4 && tiles <= (split == 2 ? res.pairs : res.quads) && k_blocks >= 8 * split; split *= 2) {
-      const double ts = start[f] + 2.0 + tile[f] + (k_blocks / split) * step[f];
-      if (ts < best_t) { best_t = ts; best = {f, split}; }
-    }
-  }
+  auto offer = [&](int f, int split, double extra) {
+    const long long row_tiles = (M + tm[f] - 1) / tm[f], tiles = batch * row_tiles * ((N + tn[f] - 1) / tn[f]);
+    const int slots = split == 4 ? res.quads : split == 2 || f <= PAIR128 ? res.pairs : res.ctas;
+    if (split > 1 && (counted || tiles > slots || k_blocks < 8 * split)) return;
+    const long long full_waves = (tiles - 1) / slots;
+    const double o = out[f] * out_scale;
+    auto wave = [&](double tiles_in_flight) {
+      const double own = step[f] + few_rows * (256.0 / tn[f] - 1.0) * tiles_in_flight / slots;
+      const double fetch = tiles_in_flight * split * tn[f] * BK * 2 / row_tiles / bytes_per_us;
+      const double products = main[f] + (k_blocks + split - 1) / split * (own > fetch ? own : fetch);
+      return products > o ? products : o;
+    };
+    const double t = start[f] + extra + full_waves * wave(slots) + wave(double(tiles - full_waves * slots)) + o;
+    if (t < best_t) { best_t = t; best = {f, split}; }
+  };
+  for (int f = 0; f < FORMS; ++f) offer(f, 1, 0.0);
+  offer(ONE64, 2, 3.7);
+  offer(ONE64, 4, 2.2);
   return best;
 }
 
@@ -754,10 +774,10 @@ static int gemm_entry(const void* A, const void* B, void* D, const void* bias, i
   p.M = M; p.N = N; p.K = K; p.ldd = ldd; p.out_fp32 = out_fp32; p.accumulate = accumulate;
   p.bias = bias; p.bias_fp32 = bias_fp32; p.D = D; p.status = jpb_status_device_ptr();
   p.counts = counts; p.seg_rows = seg_rows; p.segs = segs; p.count_k = count_k;
-  const Choice choice = choose(batch, M, N, K, counts != nullptr, resident());
+  const Choice choice = choose(batch, M, N, K, out_fp32 != 0, counts != nullptr, resident());
   const int tm = choice.form <= PAIR128 ? 256 : 128;
-  const int tn = choice.form == PAIR256 ? 256 : choice.form == ONE64 ? 64 : 128;
-  const int b_rows = choice.form == PAIR256 || choice.form == ONE128 ? 128 : 64;  // rows of B per CTA
+  const int tn = choice.form == PAIR256 || choice.form == ONE256 ? 256 : choice.form == ONE64 ? 64 : 128;
+  const int b_rows = choice.form <= PAIR128 ? tn / 2 : tn;  // rows of B per CTA
   p.tiles_m = (M + tm - 1) / tm;
   p.tiles_n = (N + tn - 1) / tn;
   p.split = choice.split;
@@ -784,6 +804,7 @@ static int gemm_entry(const void* A, const void* B, void* D, const void* bias, i
   switch (choice.form) {
     case PAIR256: return launch_layout<2, 256, false>(ma, mb, md, p, a_mn_major, b_mn_major, s);
     case PAIR128: return launch_layout<2, 128, false>(ma, mb, md, p, a_mn_major, b_mn_major, s);
+    case ONE256: return launch_layout<1, 256, false>(ma, mb, md, p, a_mn_major, b_mn_major, s);
     case ONE128: return launch_layout<1, 128, false>(ma, mb, md, p, a_mn_major, b_mn_major, s);
     default:
       if (choice.split > 1) return launch_layout<1, 64, true>(ma, mb, md, p, a_mn_major, b_mn_major, s);
@@ -793,11 +814,11 @@ static int gemm_entry(const void* A, const void* B, void* D, const void* bias, i
 
 // The form that `batch` products [M, K] x [K, N] take, and the parts of their reductions (times 16), on a device that holds
 // `ctas` CTAs, `pairs` clusters of two and `quads` of four at once (ctas = 0: this device).  Forms: 0 and 1 pairs of CTAs with
-// 256 and 128 columns, 2 and 3 single CTAs with 128 and 64.
-JPB_API int jpb_gemm_form(int batch, int M, int N, int K, int counted, int ctas, int pairs, int quads) {
+// 256 and 128 columns, 2 to 4 single CTAs with 256, 128 and 64.
+JPB_API int jpb_gemm_form(int batch, int M, int N, int K, int out_fp32, int counted, int ctas, int pairs, int quads) {
   const jpb::Resident res = ctas > 0 ? jpb::Resident{ctas, pairs, quads} : jpb::resident();
   if (res.ctas <= 0 || res.pairs <= 0 || res.quads <= 0 || batch <= 0 || M <= 0 || N <= 0 || K <= 0) return -JPB_ERR_BAD_ARGUMENT;
-  const jpb::Choice c = jpb::choose(batch, M, N, K, counted != 0, res);
+  const jpb::Choice c = jpb::choose(batch, M, N, K, out_fp32 != 0, counted != 0, res);
   return c.form + 16 * c.split;
 }
 

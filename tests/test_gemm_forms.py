@@ -4,13 +4,13 @@ import pytest
 
 from jaxpp_b200.ops import native
 
-PAIR256, PAIR128, ONE128, ONE64 = range(4)
-TILE = {PAIR256: (256, 256), PAIR128: (256, 128), ONE128: (128, 128), ONE64: (128, 64)}
+PAIR256, PAIR128, ONE256, ONE128, ONE64 = range(5)
+TILE = {PAIR256: (256, 256), PAIR128: (256, 128), ONE256: (128, 256), ONE128: (128, 128), ONE64: (128, 64)}
 CTAS, PAIRS, QUADS = 148, 74, 33
 
 
-def choice(M, N, K, batch=1, counted=False):
-    r = native.load().jpb_gemm_form(batch, M, N, K, int(counted), CTAS, PAIRS, QUADS)
+def choice(M, N, K, batch=1, counted=False, out_fp32=False):
+    r = native.load().jpb_gemm_form(batch, M, N, K, int(out_fp32), int(counted), CTAS, PAIRS, QUADS)
     return r % 16, r // 16
 
 
@@ -32,3 +32,14 @@ def test_divided_reductions_run_in_one_round(K):
                 divided.add(split)
             assert choice(M, N, K, counted=True)[1] == 1
     assert K < 4096 or divided == {2, 4}
+
+
+@pytest.mark.parametrize("M,N,K", [(77, 22016, 4096), (128, 22016, 4096), (8, 32000, 4096), (128, 28672, 1024), (384, 11008, 4096)])
+def test_wide_products_of_few_rows_take_one_round(M, N, K):
+    form, split = choice(M, N, K)
+    assert split == 1 and tiles(form, M, N) <= (CTAS if form >= ONE256 else PAIRS)
+
+
+def test_large_products_take_pairs():
+    for M, N, K in ((4096, 4096, 4096), (4096, 12288, 4096), (4096, 32000, 4096), (16384, 4096, 11008), (8192, 28672, 8192)):
+        assert choice(M, N, K) == (PAIR256, 1)
