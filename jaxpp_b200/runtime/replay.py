@@ -90,22 +90,19 @@ def _same_memory(a: torch.Tensor, b: torch.Tensor) -> bool:
     return a.data_ptr() == b.data_ptr() and a.shape == b.shape and a.stride() == b.stride() and a.dtype == b.dtype
 
 
-def _overlap(tensors: Sequence) -> bool:
-    """Do any two of these contiguous tensors share memory?"""
-    spans = sorted((x.data_ptr(), x.nbytes) for x in tensors if x is not None and x.numel())
-    return any(a + n > b for (a, n), (b, _) in zip(spans, spans[1:]))
-
-
-def _copy_all(dst: list, src: list) -> None:
-    """One multi-tensor copy per dtype."""
+def _by_dtype(tensors: Sequence, which: Sequence) -> list:
+    """Positions and tensors of ``which``, grouped for one multi-tensor copy per dtype."""
     groups: dict = {}
-    for d, s in zip(dst, src):
-        if d.numel():
-            g = groups.setdefault(d.dtype, ([], []))
-            g[0].append(d)
-            g[1].append(s)
-    for d, s in groups.values():
-        torch._foreach_copy_(d, s)
+    for k in which:
+        if tensors[k].numel():
+            g = groups.setdefault(tensors[k].dtype, ([], []))
+            g[0].append(k)
+            g[1].append(tensors[k])
+    return list(groups.values())
+
+
+def _copy(dst: list, src: list) -> None:
+    torch._foreach_copy_(dst, src)
 
 
 def _input_bytes(inputs: Sequence) -> int:
@@ -173,12 +170,33 @@ class _Recording:
                 n = len(self.results)
                 self.results.append(t)
             self.outputs.append(("out", rank, n))
+        self._plan()
         self.done.record(torch.cuda.current_stream(device))     # the first copies into the buffers
 
+    def _plan(self) -> None:
+        """What a call looks up: worked out here, since the calls are bound by the host."""
+        self.forms = [None if s is None else (s.dtype, s.shape) for s in self.static]
+        self.sizes = [0 if s is None else s.nbytes for s in self.static]
+        self.into = _by_dtype(self.static, [k for k, s in enumerate(self.static) if s is not None])
+        self.back = _by_dtype(self.static, self.written)
+        self.out = _by_dtype(self.results, range(len(self.results)))
+
     def covers(self, inputs: Sequence) -> bool:
-        """A compiled step runs on whatever tensors it is called with; the recording is one of these shapes and dtypes."""
-        return all(x is s or (x is not None and s is not None and x.dtype == s.dtype and x.shape == s.shape)
-                   for x, s in zip(inputs, self.static))
+        """A compiled step runs on whatever tensors it is called with; the recording is one of these shapes and dtypes.  A
+        step that updates an input in place is not replayed if another input sees the update: their order matters."""
+        for x, form in zip(inputs, self.forms):
+            if x is None or form is None:
+                if x is not form:
+                    return False
+            elif x.dtype != form[0] or x.shape != form[1]:
+                return False
+        if self.written:
+            end = 0
+            for a, n in sorted([(x.data_ptr(), n) for x, n in zip(inputs, self.sizes) if n]):
+                if a < end:
+                    return False
+                end = a + n
+        return True
 
     def run(self, inputs: Sequence) -> list:
         from ..ops import native
@@ -186,15 +204,16 @@ class _Recording:
         stream = torch.cuda.current_stream(self.device)
         stream.wait_event(self.done)       # the buffers may still be in use by a replay on another stream
         fresh = [torch.empty_like(t) for t in self.results]     # (if there is no memory for them, nothing has run yet)
-        live = [(s, x) for s, x in zip(self.static, inputs) if s is not None]
         try:
-            _copy_all([s for s, _ in live], [x.detach() for _, x in live])
+            for which, buffers in self.into:
+                _copy(buffers, [inputs[k] for k in which])      # (what requires grad is not replayed where grad is recorded)
             self.graph.replay()
             native.LAUNCHES[0] += self.launches
-            _copy_all(fresh, self.results)
-            if self.written:
+            for which, results in self.out:
+                _copy([fresh[n] for n in which], results)
+            for which, buffers in self.back:
                 # (.data: like the kernels' own in-place updates, this does not touch autograd's version counters)
-                _copy_all([inputs[k].data for k in self.written], [self.static[k] for k in self.written])
+                _copy([inputs[k].data for k in which], buffers)
         finally:
             self.done.record(stream)       # whatever is in flight uses the buffers, also after an error
         return [o[1] if o[0] == "c" else {o[1]: inputs[o[2]] if o[0] == "in" else fresh[o[2]]} for o in self.outputs]
@@ -205,7 +224,7 @@ class _Recording:
         except Exception:  # pragma: no cover - the context is gone at interpreter exit
             pass
         self.graph = None
-        self.static, self.results = [], []
+        self.static, self.results, self.into, self.back, self.out = [], [], [], [], []
 
 
 class StepReplay:
@@ -250,8 +269,6 @@ class StepReplay:
                 rec = self._record(inputs, device, execute)
             if rec is None or rec.settings != _settings() or rec.device != device or not rec.covers(inputs):
                 return None
-            if rec.written and _overlap(inputs):
-                return None      # an update in place of one input is seen through another: the order of the updates matters
             return rec.run(inputs)
 
     def _record(self, inputs, device, execute) -> _Recording | None:
