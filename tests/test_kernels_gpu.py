@@ -61,8 +61,7 @@ def test_gemm_wgrad_layout_and_accumulate(native, M, N, K):
     close(acc, 1.0 + 2.0 * ref, rtol=2e-2, atol=4e-2 * (M ** 0.5) * 0.25)
 
 
-# one shape or more per form of the kernel: pairs of CTAs with 256 and 128 columns, single CTAs with 128 and 64, divided
-# reductions; remainders in every dimension (N % 64 != 0 takes the unblocked MN-major copies)
+# remainders in every dimension (N % 64 != 0 takes the unblocked MN-major copies); the forms of the kernel by name are below
 @pytest.mark.parametrize("M,N,K", [(2056, 5000, 136), (4104, 1096, 264), (776, 1032, 1032), (520, 264, 72), (264, 136, 2056), (72, 4088, 4104),
                                    (8, 64, 512), (136, 8, 1544)])
 @pytest.mark.parametrize("layout", ["f", "d", "w"])
@@ -84,6 +83,86 @@ def test_gemm_forms_at_tile_edges(native, M, N, K, layout):
     wide = torch.full((M, N + 3), 7.0, dtype=torch.float32, device="cuda")   # rows that TMA cannot store; neighbours untouched
     check(run(wide[:, :N], bias=bias), ref + bias.double(), 0.0)
     assert (wide[:, N:] == 7.0).all()
+    torch.cuda.synchronize()
+    assert native.read_status(clear=False) == 0
+
+
+PAIR256, PAIR128, ONE256, ONE128, ONE64 = range(5)
+
+
+def _assert_form(native, form, split, batch, M, N, K, counted=False):
+    """(the choice goes by the number of CTAs and clusters that are resident at once: the shapes are for 148 SMs)"""
+    if torch.cuda.get_device_properties(0).multi_processor_count == 148:
+        for out_fp32 in (0, 1):
+            assert native.load().jpb_gemm_form(batch, M, N, K, out_fp32, int(counted), 0, 0, 0) == form + 16 * split
+
+
+@pytest.mark.parametrize("form,split,batch,M,N,K", [
+    (PAIR256, 1, 1, 1032, 2056, 1544), (PAIR128, 1, 1, 776, 1352, 4104), (ONE256, 1, 1, 1032, 2056, 72), (ONE128, 1, 1, 776, 1352, 72),
+    (ONE64, 1, 1, 72, 8, 72), (ONE64, 2, 1, 136, 1032, 2056), (ONE64, 4, 1, 72, 8, 2056),
+    # several problems in one launch: tiles that end in the next problem's rows
+    (PAIR256, 1, 5, 136, 2056, 2048), (PAIR256, 1, 5, 776, 2056, 1024), (PAIR128, 1, 8, 392, 1032, 4096), (ONE256, 1, 8, 136, 2056, 64),
+    (ONE128, 1, 5, 136, 1032, 64), (ONE64, 1, 2, 72, 136, 64), (ONE64, 2, 2, 136, 520, 2048), (ONE64, 4, 2, 72, 136, 2048)])
+@pytest.mark.parametrize("layout", ["f", "d", "w"])
+def test_every_gemm_form(native, form, split, batch, M, N, K, layout):
+    """Ragged shapes in each form of the kernel, all layouts, against 64 bits: bf16 and accumulated fp32 results through TMA,
+    and a result whose rows TMA cannot store.  Errors as in the test above."""
+    _assert_form(native, form, split, batch, M, N, K)
+    a = rnd(batch, *((K, M) if layout == "w" else (M, K)), seed=61)
+    b = rnd(batch, *((N, K) if layout == "f" else (K, N)), seed=62)
+    A, B = a.double(), b.double()
+    A, B = A.transpose(1, 2) if layout == "w" else A, B.transpose(1, 2) if layout == "f" else B
+    ref = A @ B
+    slack = K * 2.0 ** -23 * (A.abs() @ B.abs())
+
+    def run(out, accumulate=False):
+        if batch == 1:
+            return native.gemm(a[0], b[0], M, N, K, layout == "w", layout != "f", out[0], accumulate=accumulate)
+        return native._gemm_batched(a, b, out, batch, M, N, K, layout == "w", layout != "f", accumulate=accumulate)
+
+    def check(out, want, rounding):
+        bad = (out.double() - want).abs() > slack + rounding * want.abs() + 2.0 ** -23 * want.abs()
+        assert not bad.any(), f"{int(bad.sum())} of {bad.numel()} elements are out of bounds"
+
+    out = torch.full((batch, M, N), float("nan"), dtype=torch.bfloat16, device="cuda")
+    run(out)
+    check(out, ref, 2.0 ** -8)
+    out = torch.full((batch, M, N), 3.0, device="cuda")
+    run(out, accumulate=True)
+    check(out, ref + 3, 0.0)
+    wide = torch.full((batch, M, N + 3), 7.0, device="cuda")      # neighbours untouched
+    run(wide[:, :, :N])
+    check(wide[:, :, :N], ref, 0.0)
+    assert (wide[:, :, N:] == 7.0).all()
+    torch.cuda.synchronize()
+    assert native.read_status(clear=False) == 0
+
+
+@pytest.mark.parametrize("form,batch,M,N,K,segs", [(PAIR256, 5, 776, 2056, 1024, 2), (PAIR256, 5, 776, 2056, 1024, 8), (PAIR128, 8, 392, 1032, 4096, 2),
+                                                   (ONE256, 8, 136, 2056, 64, 2), (ONE128, 5, 136, 1032, 64, 1), (ONE64, 3, 72, 136, 64, 1)])
+@pytest.mark.parametrize("layout", ["f", "d", "w"])
+def test_every_gemm_form_with_row_counts(native, form, batch, M, N, K, segs, layout):
+    """Groups that fill only the first rows of each segment: empty tiles of every height are skipped and written as zeros, or
+    left alone when the result is added, and so are empty blocks of a reduction (layout w)."""
+    _assert_form(native, form, 1, batch, M, N, K, counted=True)
+    over_k = layout == "w"
+    if over_k:
+        segs = max(1, segs // 2)
+    seg = (K if over_k else M) // segs
+    counts = torch.randint(0, seg + 1, (batch, segs), generator=torch.Generator().manual_seed(9), dtype=torch.int32)
+    counts[0], counts[1], counts[2, 0] = seg, 0, 1
+    live = (torch.arange(seg)[None, None] < counts[:, :, None]).reshape(batch, seg * segs, 1).cuda()
+    a = rnd(batch, *((K, M) if over_k else (M, K)), seed=61) * live
+    b = rnd(batch, *((N, K) if layout == "f" else (K, N)), seed=62)
+    A, B = a.double(), b.double()
+    A, B = A.transpose(1, 2) if over_k else A, B.transpose(1, 2) if layout == "f" else B
+    ref = A @ B
+    slack = K * 2.0 ** -23 * (A.abs() @ B.abs())
+    run = lambda out, acc: native._gemm_batched(a, b, out, batch, M, N, K, over_k, layout != "f", counts.cuda(), seg, over_k, acc)
+    out = run(torch.full((batch, M, N), float("nan"), dtype=torch.bfloat16, device="cuda"), False)
+    assert ((out.double() - ref).abs() <= slack + 2.0 ** -8 * ref.abs()).all()
+    out = run(torch.full((batch, M, N), 3.0, device="cuda"), True)
+    assert ((out.double() - ref - 3).abs() <= slack + 2.0 ** -23 * (ref + 3).abs()).all()
     torch.cuda.synchronize()
     assert native.read_status(clear=False) == 0
 
