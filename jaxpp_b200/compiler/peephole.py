@@ -3,11 +3,13 @@
 ``fuse_norm_backward_adds``: in a pre-norm residual block the gradient of the block input is the sum of the
 normalisation's input gradient and the gradient that arrives over the residual connection.  Autograd emits that as
 ``norm_bwd`` followed by an ``add`` kernel that re-reads both tensors; the fused op writes the sum in the pass that
-produces the first operand.  The sum is rounded exactly as the two separate kernels would round it, so a rewritten
-program still matches the eager step bit for bit.
+produces the first operand.  The sum is rounded exactly as the two separate kernels would round it: this rewrite leaves a
+program's results as they are, bit for bit.
 
 ``widen_parameter_sums``: with fp32 gradients the sums that are the gradients of biases and norm weights are produced in
-the parameters' type and cast by a kernel of their own each.  The ops can leave their fp32 sums as they are.
+the parameters' type and cast by a kernel of their own each.  The ops can leave their fp32 sums as they are.  A program
+that gets this rewrite is more exact than the eager step, whose sums are rounded to the parameters' type in between, and no
+longer the same bits.
 """
 from __future__ import annotations
 

@@ -1,7 +1,7 @@
 // Tensor-parallel GEMMs fused with their collective over NVLink peer memory (sm_100a).
 //
-// One persistent kernel per op; the tcgen05 main loop is the one of gemm_sm100.cu (TMA ring -> tcgen05.mma
-// -> double-buffered TMEM accumulators -> epilogue warps) plus four "comm" warps per CTA.
+// One persistent kernel per op; the tcgen05 main loop works on 128 x 256 tiles of one CTA (TMA ring -> tcgen05.mma
+// -> double-buffered TMEM accumulators -> epilogue warps; gemm_sm100.cu has others), plus four "comm" warps per CTA.
 //
 //  all-gather -> GEMM   Every rank owns a symmetric buffer G[n_ranks][rows_per_rank, width].  The comm warps
 //                       of rank r PUSH r's shard straight from the tensor it lives in into slot r of every
