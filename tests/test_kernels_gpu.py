@@ -658,6 +658,10 @@ def test_flash_attention_at_block_edges(native, B, Sq, Sk, H, Hkv, causal, D):
     """Pairs of query tiles of which one is empty or short, single and odd numbers of blocks, fully hidden rows, against
     64 bits.  P and dS are rounded to bf16 before the second products (2^-9 each) and the results once more, so each
     result is within 3 * 2^-8 of its 2-norm; the log-sum-exp is all fp32."""
+    _check_attention(native, B, Sq, Sk, H, Hkv, causal, D)
+
+
+def _check_attention(native, B, Sq, Sk, H, Hkv, causal, D):
     q, k, v, do = rnd(B, Sq, H, D, seed=71), rnd(B, Sk, Hkv, D, seed=72), rnd(B, Sk, Hkv, D, seed=73), rnd(B, Sq, H, D, seed=74)
     scale, G = D ** -0.5, H // Hkv
     o, lse = native.attention(q, k, v, causal, scale)
@@ -678,6 +682,43 @@ def test_flash_attention_at_block_edges(native, B, Sq, Sk, H, Hkv, causal, D):
         assert (a.double() - b).norm() <= 3 * 2.0 ** -8 * b.norm()
     torch.cuda.synchronize()
     assert native.read_status(clear=False) == 0
+
+
+# grids with more pairs of tiles than SMs take two tiles per CTA, smaller ones the two halves of one tile
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("halves,B,Sq,Sk,H,Hkv,causal", [
+    (0, 75, 250, 506, 4, 2, True), (0, 80, 130, 391, 4, 4, False), (0, 100, 300, 100, 2, 2, True), (0, 2, 128, 128, 4, 4, True),
+    (0, 72, 200, 3, 2, 1, False), (1, 1, 1025, 1025, 4, 2, True), (1, 3, 129, 1153, 2, 2, False), (1, 2, 257, 129, 2, 1, True),
+    (1, 1, 64, 193, 2, 2, False), (1, 1, 300, 257, 4, 4, True), (1, 2, 300, 100, 2, 1, True)])
+def test_flash_attention_in_both_forms(native, halves, B, Sq, Sk, H, Hkv, causal, D):
+    """Odd and even numbers of blocks (the halves keep two blocks of scores), last blocks with nothing in the second half, tiles
+    behind the last query, rows that see no key."""
+    if torch.cuda.get_device_properties(0).multi_processor_count == 148:
+        assert native.load().jpb_attention_fwd_halves(B, Sq, Sk, H, D, int(causal)) == halves
+    _check_attention(native, B, Sq, Sk, H, Hkv, causal, D)
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("where", ["first", "second", "both", "apart"])
+def test_flash_attention_halves_rescale(native, D, where):
+    """Scores whose maximum grows block by block in one half of the keys, in the other, or in both, or that are far lower in
+    one half everywhere: each half rescales its sums on its own, and the halves meet with maxima far apart."""
+    B, S, H = 1, 1280, 2
+    if torch.cuda.get_device_properties(0).multi_processor_count == 148:
+        assert native.load().jpb_attention_fwd_halves(B, S, S, H, D, 1) == 1
+    col = torch.arange(S, device="cuda")
+    first, ramp = ((col % 128) < 64).float(), (1 + col // 128).float()
+    gain = {"first": first * ramp, "second": (1 - first) * ramp, "both": ramp, "apart": 20 * first - 10}[where]
+    q, v = rnd(B, S, H, D, seed=75).abs(), rnd(B, S, H, D, seed=77)
+    k = (rnd(B, S, H, D, seed=76).float() * 0.3 + 0.5 * gain[None, :, None, None]).to(torch.bfloat16)
+    o, lse = native.attention(q, k, v, True, D ** -0.5)
+    s = torch.einsum("bqhd,bkhd->bhqk", q.double(), k.double()) * D ** -0.5
+    s = s.masked_fill(col[None, :] > col[:, None], float("-inf"))
+    rlse = torch.logsumexp(s, -1)
+    ro = torch.einsum("bhqk,bkhd->bqhd", torch.exp(s - rlse[..., None]), v.double())
+    assert float((s[0, 0, -1].max() - s[0, 0, -1].min())) > 20      # far more than the 8 steps of log2 that move a maximum
+    close(lse, rlse.float(), rtol=1e-5, atol=1e-5)
+    assert (o.double() - ro).norm() <= 3 * 2.0 ** -8 * ro.norm()
 
 
 @pytest.mark.parametrize("rows,H,per_sm", [(3000, 2048, 2), (6000, 1024, 4), (7200, 1024, 8), (3600, 1600, 4), (9000, 4096, 2)])
