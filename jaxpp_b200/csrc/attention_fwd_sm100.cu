@@ -11,8 +11,8 @@
 // tile's softmax could overlap its own products, which depend on it; with two tiles in turn the tensor cores work on
 // one while the exponentials of the other are taken.  A thread per row needs no exchange of maxima between warps.
 // O is rescaled in TMEM only when some row's maximum has moved by enough to matter.
-// Causal, 32 heads of 128: 4096 rows 148 us (927 TFLOP/s), 16384 rows 2.02 ms (1089); with one tile per CTA and its
-// columns split among four warp groups, all in step with each other, 226 us and 2.63 ms.
+// Causal, 32 heads of 128: 4096 rows 140 us (980 TFLOP/s), 16384 rows 1.88 ms (1170); with one tile per CTA and its
+// columns split among four warp groups, all in step with each other, 224 us and 2.63 ms.
 //
 // HALVES is for grids that leave SMs without a pair of tiles: the two softmax groups take the first and the second 64 keys of
 // every block as two independent sums over the same tile, which meet at the end.  Two buffers for the scores of a half let S
@@ -461,11 +461,13 @@ static int launch_attn_fwd(const void* q, const void* k, const void* v, const At
   return int(cudaGetLastError());
 }
 
-// Which of the two forms?  Estimated time of each in steps of one block: two tiles in turn take 1.93 us a block at head_dim
-// 128 (1.78 at 64), the halves of one tile 1.36 (1.08), and a CTA three to four blocks' time to start and end.  Where tiles
-// differ in length (causal), the long ones start first and the short ones fill the gaps; else the CTAs run in whole rounds.
-// Two rounds of halves are slower than one of pairs: 25 heads of 128, 1024 rows, all keys: 32 against 25 us; causal 19 against 24.
-// With a single block and tile there is nothing to overlap, and the halves' meeting costs 3 to 6 %.
+// Which of the two forms?  Estimated times: two tiles in turn take 1.93 us a block at head_dim 128 (1.78 at 64), the halves of
+// one tile 1.36 (1.08), and a CTA 4 us to start and end.  Where tiles differ in length (causal), the long ones start first and
+// the short ones fill the gaps but for 5 %; else the CTAs run in whole rounds.  Of 179 grids measured in both forms (head_dim
+// 64 and 128, 1 to 64 heads, 1 to 16384 rows) the estimate's choice is more than 3 % slower than the other in two, by 5 %.
+// Two rounds of halves are slower than one of pairs: 25 heads of 128, 1024 rows, all keys: 32 against 25 us; causal 19 against
+// 24; 16 x 8 heads of 512 causal rows 32 against 26.
+// With a single block and tile there is nothing to overlap; which form is faster goes by 0.4 us either way.
 static bool halves_are_faster(const AttnParams& p, int D) {
   if (p.Sk <= ATT_BN && p.Sq <= ATT_BM) return false;
   static const int sms = [] {
@@ -483,10 +485,10 @@ static bool halves_are_faster(const AttnParams& p, int D) {
       most = n > most ? n : most;
       least = n < least ? n : least;
     }
-    const double ends = 3.5;
-    if (2 * least >= most) return step * double((ctas * heads + sms - 1) / sms) * (most + ends);
-    const double shared = double(heads) * (total + ends * ctas) / sms;
-    return step * (shared > most + ends ? shared : most + ends);
+    const double ends = 4.0, longest = most * step + ends;
+    if (least == most) return double((ctas * heads + sms - 1) / sms) * longest;
+    const double shared = 1.05 * heads * (total * step + ends * ctas) / sms;
+    return shared > longest ? shared : longest;
   };
   return time(ATT_BM, D == 128 ? 1.36 : 1.08) < time(2 * ATT_BM, D == 128 ? 1.93 : 1.78);
 }
